@@ -65,6 +65,7 @@ struct TcArgs {
   int pack16;                      /* bfloat16 result, N and the row pitch multiples of 8, addend absent or one value per column:
                                       bias, activation and rounding happen in registers and the staged tile holds bfloat16 */
   int tiles_m, tiles_n, n_tiles;   /* n_tiles = nbatch * tiles_m * tiles_n */
+  int a_mn, b_mn;                  /* the operand's rows are contiguous and k is strided (16-bit elements): staged as stored */
   int m_fast;                      /* consecutive tiles differ in the row tile (else in the column tile) */
   int kchunk;                      /* PROMOTE kernels: k-blocks summed in tensor memory before the partial sum moves to registers */
   float alpha;                     /* PROMOTE kernels: the sum is scaled by this before the addend (a parameter update behind a gradient) */
@@ -134,7 +135,11 @@ struct TcSmem {
   static constexpr int BYTES = STAGES * STAGE + EPI + 256 + 1024; /* + barriers + alignment slack */
 };
 
-template <int BN, int CTAS, bool PROMOTE = false, bool TF32 = false>
+#define MN_BOX 8192              /* bytes of a box of 64 k x 64 contiguous rows of 16-bit elements */
+
+/* MN: an operand may have contiguous rows (a_mn, b_mn); without it the kernel is compiled for k-contiguous ones alone,
+ * which keeps the issuing threads of short contractions free of the choice (197 x 2304 x 768: 1 us). */
+template <int BN, int CTAS, bool PROMOTE = false, bool TF32 = false, bool MN = false>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 pb200_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const TcArgs g) {
   using S = TcSmem<BN, CTAS>;
@@ -198,12 +203,17 @@ pb200_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
             /* both CTAs' bytes are counted on the first CTA's barrier, whose MMA thread waits for them */
             const uint32_t full0 = mapa_shared(bar_full + 8 * stage, 0);
             if (rank == 0) mbar_expect_tx(bar_full + 8 * stage, 2 * S::STAGE);
-            tma_load_3d_pair(sa, &map_a, full0, kb * bk, (mt * 2 + (int)rank) * TC_BM, bz);
-            tma_load_3d_pair(sb, &map_b, full0, kb * bk, nt * BN + (int)rank * (BN / 2), bz);
+            const int ra = (mt * 2 + (int)rank) * TC_BM, rb = nt * BN + (int)rank * (BN / 2);
+            if (MN && g.a_mn) for (int i = 0; i < TC_BM / 64; i++) tma_load_3d_pair(sa + i * MN_BOX, &map_a, full0, ra + i * 64, kb * bk, bz);
+            else tma_load_3d_pair(sa, &map_a, full0, kb * bk, ra, bz);
+            if (MN && g.b_mn) for (int i = 0; i < BN / 2 / 64; i++) tma_load_3d_pair(sb + i * MN_BOX, &map_b, full0, rb + i * 64, kb * bk, bz);
+            else tma_load_3d_pair(sb, &map_b, full0, kb * bk, rb, bz);
           } else {
             mbar_expect_tx(bar_full + 8 * stage, S::STAGE);
-            tma_load_3d(sa, &map_a, bar_full + 8 * stage, kb * bk, mt * TC_BM, bz);
-            tma_load_3d(sb, &map_b, bar_full + 8 * stage, kb * bk, nt * BN, bz);
+            if (MN && g.a_mn) for (int i = 0; i < TC_BM / 64; i++) tma_load_3d(sa + i * MN_BOX, &map_a, bar_full + 8 * stage, mt * TC_BM + i * 64, kb * bk, bz);
+            else tma_load_3d(sa, &map_a, bar_full + 8 * stage, kb * bk, mt * TC_BM, bz);
+            if (MN && g.b_mn) for (int i = 0; i < BN / 64; i++) tma_load_3d(sb + i * MN_BOX, &map_b, bar_full + 8 * stage, nt * BN + i * 64, kb * bk, bz);
+            else tma_load_3d(sb, &map_b, bar_full + 8 * stage, kb * bk, nt * BN, bz);
           }
           if (++stage == S::STAGES) { stage = 0; phase ^= 1u; }
         }
@@ -212,26 +222,29 @@ pb200_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
   } else if (warp == 1) {
     /* ── MMA issuer ── */
     if (lane == 0 && rank == 0) {
-      /* D float32; A and B float16 (format 0), bfloat16 (1) or tf32 (2, a compile-time variant), both
-       * K-major.  A tile row is 128 bytes in every format and one instruction consumes 32 of them
-       * (16 or 8 elements). */
+      /* D float32; A and B float16 (format 0), bfloat16 (1) or tf32 (2, a compile-time variant).  K-major: a
+       * tile row is 128 bytes in every format and one instruction consumes 32 of them (16 or 8 elements).
+       * Rows contiguous (bits 15 and 16): a box holds 64 k of 64 rows, 128 bytes each, and one
+       * instruction consumes 16 k, two 1024-byte groups. */
       const uint32_t fmt = TF32 ? 2u : (uint32_t)g.ab_fmt;
-      const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((TC_BM * CTAS) >> 4) << 24);
+      const bool a_mn = MN && g.a_mn, b_mn = MN && g.b_mn;
+      const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((a_mn ? 1u : 0u) << 15) | ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((TC_BM * CTAS) >> 4) << 24);
+      const uint64_t ka = a_mn ? 128 : 2, kb = b_mn ? 128 : 2;      /* descriptor units (16 bytes) from one instruction's k to the next's */
       uint32_t stage = 0, phase = 0, it = 0;
       bool ok = true;
       /* the four instructions of one k-block; `first` clears the accumulator */
       auto issue_block = [&](uint32_t tmem_d, bool first) {
         const uint32_t sa = base + stage * S::STAGE, sb = sa + S::STAGE_A;
-        const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sb);
+        const uint64_t da = a_mn ? make_smem_desc_mn(sa, MN_BOX) : make_smem_desc(sa), db = b_mn ? make_smem_desc_mn(sb, MN_BOX) : make_smem_desc(sb);
 #pragma unroll
         for (int k = 0; k < TC_BK / 16; k++) {
           const uint32_t accum = (!first || k) ? 1u : 0u;
           if constexpr (CTAS == 2) {
-            if constexpr (TF32) tc_mma_tf32_pair(tmem_d, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, accum);
-            else tc_mma_bf16_pair(tmem_d, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, accum);
+            if constexpr (TF32) tc_mma_tf32_pair(tmem_d, da + k * ka, db + k * kb, idesc, accum);
+            else tc_mma_bf16_pair(tmem_d, da + k * ka, db + k * kb, idesc, accum);
           } else {
-            if constexpr (TF32) tc_mma_tf32(tmem_d, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, accum);
-            else tc_mma_bf16(tmem_d, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, accum);
+            if constexpr (TF32) tc_mma_tf32(tmem_d, da + k * ka, db + k * kb, idesc, accum);
+            else tc_mma_bf16(tmem_d, da + k * ka, db + k * kb, idesc, accum);
           }
         }
         /* frees the stage (in both CTAs of a pair) when these MMAs have read it */
@@ -245,10 +258,10 @@ pb200_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
           if (!mbar_wait(bar_tempty + 8 * buf, (use & 1u) ^ 1u, &abort_flag, 2)) { ok = false; break; }
           tc_fence_after_sync();
           const uint32_t tmem_d = tmem_base + buf * BN;
-          for (int kb = 0; kb < kblocks; kb++) {
+          for (int kblk = 0; kblk < kblocks; kblk++) {
             if (!mbar_wait(bar_full + 8 * stage, phase, &abort_flag, 3)) { ok = false; break; }
             tc_fence_after_sync();
-            issue_block(tmem_d, kb == 0);
+            issue_block(tmem_d, kblk == 0);
           }
           if (ok) { if constexpr (CTAS == 2) tc_commit_pair(bar_tfull + 8 * buf, 3); else tc_commit(bar_tfull + 8 * buf); }   /* accumulator complete */
         }
@@ -263,10 +276,10 @@ pb200_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
             tc_fence_after_sync();
             const uint32_t tmem_d = tmem_base + buf * BN;
             const int kend = min(kb0 + g.kchunk, kblocks);
-            for (int kb = kb0; kb < kend; kb++) {
+            for (int kblk = kb0; kblk < kend; kblk++) {
               if (!mbar_wait(bar_full + 8 * stage, phase, &abort_flag, 3)) { ok = false; break; }
               tc_fence_after_sync();
-              issue_block(tmem_d, kb == kb0);
+              issue_block(tmem_d, kblk == kb0);
             }
             if (ok) tc_commit(bar_tfull + 8 * buf);
           }
@@ -604,11 +617,11 @@ static int make_map(CUtensorMap *map, const void *ptr, long long K, long long ro
 }
 
 /* One-time set-up of a kernel variant (the runtime drives one device per process). */
-template <int BN, int CTAS, bool PROMOTE = false, bool TF32 = false>
+template <int BN, int CTAS, bool PROMOTE = false, bool TF32 = false, bool MN = false>
 static int tc_configure() {
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(pb200_gemm_tc<BN, CTAS, PROMOTE, TF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcSmem<BN, CTAS>::BYTES);
+    cudaError_t e = cudaFuncSetAttribute(pb200_gemm_tc<BN, CTAS, PROMOTE, TF32, MN>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcSmem<BN, CTAS>::BYTES);
     if (e != cudaSuccess) { pb_set_error("gemm: cannot reserve %d bytes of shared memory: %s", TcSmem<BN, CTAS>::BYTES, cudaGetErrorString(e)); return -1; }
     configured = true;
   }
@@ -621,9 +634,9 @@ static int sm_count() {
   return sms;
 }
 
-template <int BN, int CTAS, bool PROMOTE = false, bool TF32 = false>
+template <int BN, int CTAS, bool PROMOTE = false, bool TF32 = false, bool MN = false>
 static int tc_launch(const CUtensorMap &ma, const CUtensorMap &mb, TcArgs &g, long long nbatch, cudaStream_t stream) {
-  if (tc_configure<BN, CTAS, PROMOTE, TF32>() != 0) return -1;
+  if (tc_configure<BN, CTAS, PROMOTE, TF32, MN>() != 0) return -1;
   g.tiles_m = (g.M + TC_BM * CTAS - 1) / (TC_BM * CTAS);
   g.tiles_n = (g.N + BN - 1) / BN;
   long long tiles = (long long)g.tiles_m * g.tiles_n * nbatch;
@@ -638,7 +651,7 @@ static int tc_launch(const CUtensorMap &ma, const CUtensorMap &mb, TcArgs &g, lo
   const int grid = (int)(tiles < units ? tiles : units) * CTAS;
   cudaError_t e;
   if (CTAS == 1) {
-    pb200_gemm_tc<BN, CTAS, PROMOTE, TF32><<<grid, TC_THREADS, TcSmem<BN, CTAS>::BYTES, stream>>>(ma, mb, g);
+    pb200_gemm_tc<BN, CTAS, PROMOTE, TF32, MN><<<grid, TC_THREADS, TcSmem<BN, CTAS>::BYTES, stream>>>(ma, mb, g);
     e = cudaGetLastError();
   } else {
     cudaLaunchConfig_t cfg = {};
@@ -647,10 +660,19 @@ static int tc_launch(const CUtensorMap &ma, const CUtensorMap &mb, TcArgs &g, lo
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = CTAS; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, pb200_gemm_tc<BN, CTAS, PROMOTE, TF32>, ma, mb, g);
+    e = cudaLaunchKernelEx(&cfg, pb200_gemm_tc<BN, CTAS, PROMOTE, TF32, MN>, ma, mb, g);
   }
   if (e != cudaSuccess) { pb_set_error("tensor-core gemm launch: %s", cudaGetErrorString(e)); return -1; }
   return 0;
+}
+
+template <bool MN>
+static int tc_launch_16(int BN, int ctas, const CUtensorMap &ma, const CUtensorMap &mb, TcArgs &g, long long nbatch, cudaStream_t stream) {
+  if (ctas == 2) return tc_launch<256, 2, false, false, MN>(ma, mb, g, nbatch, stream);
+  if (BN == 256) return tc_launch<256, 1, false, false, MN>(ma, mb, g, nbatch, stream);
+  if (BN == 192) return tc_launch<192, 1, false, false, MN>(ma, mb, g, nbatch, stream);
+  if (BN == 128) return tc_launch<128, 1, false, false, MN>(ma, mb, g, nbatch, stream);
+  return tc_launch<64, 1, false, false, MN>(ma, mb, g, nbatch, stream);
 }
 
 int pb_gemm_tc_error(void) {
@@ -885,7 +907,7 @@ static const void *tc_operand_x3(PbGemmProgram &p, PbTcOperand &cache, const voi
 
 /* A bf16 operand that is already K-major with 16-byte aligned rows is read in
  * place by TMA; anything else goes through tc_operand. */
-struct TcView { const void *ptr; long long pitch, bpitch; };
+struct TcView { const void *ptr; long long pitch, bpitch; bool mn = false; };
 
 static bool tc_in_place(const PbGemmProgram &p, const void *buf, long long off, bool is_a, TcView *v) {
   if (p.dtype == PB_F32 && !(is_a && p.a_bf16)) return false;
@@ -898,6 +920,23 @@ static bool tc_in_place(const PbGemmProgram &p, const void *buf, long long off, 
   const char *ptr = (const char *)buf + off * 2;
   if ((reinterpret_cast<uintptr_t>(ptr) & 15) || pitch % 8 || pitch < p.K || (p.nbatch > 1 && (bp % 8 || bp <= 0))) return false;
   v->ptr = ptr; v->pitch = pitch; v->bpitch = bp;
+  return true;
+}
+
+/* A 16-bit operand whose rows (m or n) are contiguous and whose k is strided -- the weights of a plain matmul,
+ * the activations of a weight gradient -- is read in place too: the tensor cores take either order, TMA only
+ * wants the k stride to be a multiple of 16 bytes.  (Copied into k order first, 4096 x 4096 x 4096 took 206 us,
+ * of which the product was 97; 8192 x 3072 x 768 with GELU 62, of which 44.) */
+static bool tc_in_place_mn(const PbGemmProgram &p, const void *buf, long long off, bool is_a, TcView *v) {
+  if (p.dtype == PB_F32) return false;
+  const bool direct = is_a ? p.a_direct : p.b_direct;
+  const long long sk = is_a ? p.a_sk : p.b_sk, srow = is_a ? p.a_sm : p.b_sn;
+  const long long rows = is_a ? p.M : p.N;
+  if (!direct || srow != 1 || p.b_ax.size() > 1) return false;
+  long long bp = p.b_ax.empty() ? p.K * sk : (is_a ? p.b_ax[0].sa : p.b_ax[0].sb);
+  const char *ptr = (const char *)buf + off * 2;
+  if ((reinterpret_cast<uintptr_t>(ptr) & 15) || sk % 8 || sk < rows || (p.nbatch > 1 && (bp % 8 || bp <= 0))) return false;
+  v->ptr = ptr; v->pitch = sk; v->bpitch = bp; v->mn = true;
   return true;
 }
 
@@ -938,10 +977,12 @@ int pb_gemm_tc_run(PbGemmProgram &p, void *const *bufs, cudaStream_t stream, int
     vb.pitch = 3 * Kp; vb.bpitch = p.N * 3 * Kp;
   } else if (!tc_in_place(p, bufs[p.p_a], p.off_a, true, &va)) {
     if (p.a_bf16) { pb_set_error("gemm: bfloat16 A operand is not addressable in place (alignment)"); return -1; }
+    if (!tc_in_place_mn(p, bufs[p.p_a], p.off_a, true, &va)) {
     va.ptr = tc_operand(p, p.tc_a, bufs[p.p_a], p.off_a, true, p.M, Kp, stream, &scr_a);
     va.pitch = Kp; va.bpitch = p.M * Kp;
+    }
   }
-  if (!fp32x3 && va.ptr && !tc_in_place(p, bufs[p.p_b], p.off_b, false, &vb)) {
+  if (!fp32x3 && va.ptr && !tc_in_place(p, bufs[p.p_b], p.off_b, false, &vb) && !tc_in_place_mn(p, bufs[p.p_b], p.off_b, false, &vb)) {
     vb.ptr = tc_operand(p, p.tc_b, bufs[p.p_b], p.off_b, false, p.N, Kp, stream, &scr_b);
     vb.pitch = Kp; vb.bpitch = p.N * Kp;
   }
@@ -1024,8 +1065,11 @@ int pb_gemm_tc_run(PbGemmProgram &p, void *const *bufs, cudaStream_t stream, int
     if (c && atoi(c) == 2) { ctas = 2; BN = 256; }
   }
   CUtensorMap ma, mb;
-  int rc = make_map(&ma, va.ptr, g.K, rowsA, p.nbatch, va.pitch, va.bpitch, TC_BM, g.ab_fmt);
-  if (rc == 0) rc = make_map(&mb, vb.ptr, g.K, rowsB, p.nbatch, vb.pitch, vb.bpitch, BN / ctas, g.ab_fmt);
+  g.a_mn = va.mn; g.b_mn = vb.mn;
+  int rc = va.mn ? make_map(&ma, va.ptr, rowsA, g.K, p.nbatch, va.pitch, va.bpitch, TC_BK, g.ab_fmt)
+                 : make_map(&ma, va.ptr, g.K, rowsA, p.nbatch, va.pitch, va.bpitch, TC_BM, g.ab_fmt);
+  if (rc == 0) rc = vb.mn ? make_map(&mb, vb.ptr, rowsB, g.K, p.nbatch, vb.pitch, vb.bpitch, TC_BK, g.ab_fmt)
+                          : make_map(&mb, vb.ptr, g.K, rowsB, p.nbatch, vb.pitch, vb.bpitch, BN / ctas, g.ab_fmt);
   if (rc != 0) { pb_scratch_free(scr_a); pb_scratch_free(scr_b); return -1; }
   pb_tc_mark_used();
   pb_tc_configure_backoff();
@@ -1044,11 +1088,8 @@ int pb_gemm_tc_run(PbGemmProgram &p, void *const *bufs, cudaStream_t stream, int
     else if (BN == 128) rc = tc_launch<128, 1, false, true>(ma, mb, g, p.nbatch, stream);
     else rc = tc_launch<64, 1, false, true>(ma, mb, g, p.nbatch, stream);
   }
-  else if (ctas == 2) rc = tc_launch<256, 2>(ma, mb, g, p.nbatch, stream);
-  else if (BN == 256) rc = tc_launch<256, 1>(ma, mb, g, p.nbatch, stream);
-  else if (BN == 192) rc = tc_launch<192, 1>(ma, mb, g, p.nbatch, stream);
-  else if (BN == 128) rc = tc_launch<128, 1>(ma, mb, g, p.nbatch, stream);
-  else rc = tc_launch<64, 1>(ma, mb, g, p.nbatch, stream);
+  else if (va.mn || vb.mn) rc = tc_launch_16<true>(BN, ctas, ma, mb, g, p.nbatch, stream);
+  else rc = tc_launch_16<false>(BN, ctas, ma, mb, g, p.nbatch, stream);
   p.launches++;
   /* stream-ordered pool: later work on this stream may reuse the blocks */
   pb_scratch_free(scr_a); pb_scratch_free(scr_b);

@@ -169,6 +169,11 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
   d |= (uint64_t)2 << 61;                 /* 128-byte swizzle */
   return d;
 }
+/* Rows contiguous ("MN-major"): 64 rows (128 bytes, swizzled) per k, eight k per 1024 bytes; the next 64 rows
+ * are `group` bytes on. */
+__device__ __forceinline__ uint64_t make_smem_desc_mn(uint32_t saddr, uint32_t group) {
+  return (make_smem_desc(saddr) & ~((uint64_t)0x3fff << 16)) | (uint64_t)(group >> 4) << 16;
+}
 
 
 /* Host side: the including file's copy of the back-off threshold, set once from the environment. */

@@ -1,0 +1,59 @@
+"""Contractions through the C entry points with each operand stored either way round, at the edges of
+tiles, of 64-row boxes and of k blocks, with row pitches TMA can and cannot address, against float64.
+
+16-bit products are exact and summed in float32: the error of a sum of K terms is below K 2^-24 of the
+sum of their magnitudes, for these sizes and random signs far below 1e-5 of the result's rms times ten."""
+import numpy as np
+import pytest
+
+from conftest import assert_close
+from kernel_lib import kernels  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+def bf16(x):
+    """Rounded to nearest even, as float32."""
+    u = np.ascontiguousarray(x, np.float32).view(np.uint32)
+    return ((u + 0x7fff + ((u >> 16) & 1)) & np.uint32(0xffff0000)).view(np.float32)
+
+
+def bits(x):
+    return (np.ascontiguousarray(x, np.float32).view(np.uint32) >> 16).astype(np.uint16)
+
+
+def stored(x, kfast, pad, rng, conv):
+    """The matrix x [rows][k] in memory: k fastest, or rows fastest; `pad` unused elements after each line."""
+    m = x if kfast else x.T
+    buf = np.full((m.shape[0], m.shape[1] + pad), np.nan, np.float32)
+    buf[:, :m.shape[1]] = m
+    ld = buf.shape[1]
+    return conv(buf), ((ld, 1) if kfast else (1, ld))
+
+
+SIZES = [(128, 64, 64), (1, 8, 16), (40, 72, 24), (197, 200, 768), (130, 257, 100), (64, 264, 1032), (300, 136, 17)]
+
+
+@pytest.mark.parametrize('pad', [0, 8, 3])
+@pytest.mark.parametrize('a_kfast,b_kfast', [(True, False), (True, True), (False, False), (False, True)])
+@pytest.mark.parametrize('m,n,k', SIZES, ids=str)
+def test_bf16_operands(kernels, m, n, k, a_kfast, b_kfast, pad):  # noqa: F811
+    run_bf16(kernels, m, n, k, a_kfast, b_kfast, pad)
+
+
+@pytest.mark.parametrize('a_kfast,b_kfast', [(True, False), (False, False), (False, True)])
+def test_bf16_operands_of_cta_pairs(kernels, a_kfast, b_kfast):  # noqa: F811
+    """Enough 256 x 256 tiles and k for CTA pairs, with a remainder on every axis."""
+    run_bf16(kernels, 2312, 2184, 1048, a_kfast, b_kfast, 0)
+
+
+def run_bf16(kernels, m, n, k, a_kfast, b_kfast, pad):  # noqa: F811
+    rng = np.random.default_rng([m, n, k, pad])
+    a, b = bf16(rng.standard_normal((m, k))), bf16(rng.standard_normal((n, k)))
+    bias = rng.standard_normal(n).astype(np.float32)
+    ma, (a_sm, a_sk) = stored(a, a_kfast, pad, rng, bits)
+    mb, (b_sn, b_sk) = stored(b, b_kfast, pad, rng, bits)
+    c = kernels.put(np.zeros((m, n), np.float32))
+    assert kernels.c.poly_b200_gemm(m, n, k, kernels.put(ma), a_sm, a_sk, kernels.put(mb), b_sk, b_sn, c, n, kernels.put(bias), 0, 1) == 0, kernels.error()
+    want = a.astype(np.float64) @ b.T.astype(np.float64) + bias
+    assert_close(kernels.get(c, (m, n)), want, 1e-4, f'bf16 {m} {n} {k}')
