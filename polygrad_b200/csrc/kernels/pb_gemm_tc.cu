@@ -57,6 +57,7 @@ struct TcArgs {
   int M, N, K;
   long long c_sm, x_sm, x_sn;
   int nb; int bext[4]; long long c_sb[4], x_sb[4];
+  int nbatch;                      /* tf32: the lo parts of batch entry z are entry z + nbatch of the operands' maps */
   int has_x, relu;
   int ab_fmt;                      /* operand format: 0 float16, 1 bfloat16 (64 per 128-byte tile row), 2 tf32 (32 per row) */
   int vec_io;                      /* C rows (and addend rows) 16-byte aligned, N % 4 == 0 */
@@ -125,12 +126,13 @@ __device__ __forceinline__ void tile_coords(const TcArgs &g, int t, int *mt, int
 
 /* CTAS = 2: two CTAs on neighbouring SMs (a cluster of 2) work on one 256 x BN tile with
  * cta_group::2 MMAs; each holds its 128 rows of A and half of the tile's B rows. */
-template <int BN, int CTAS>
+template <int BN, int CTAS, bool TF32 = false>
 struct TcSmem {
-  static constexpr int STAGE_A = TC_BM * TC_BK * 2;
-  static constexpr int STAGE_B = (BN / CTAS) * TC_BK * 2;
+  static constexpr int PARTS = TF32 ? 2 : 1;                 /* a float32 operand comes as two tf32 tiles, hi and lo */
+  static constexpr int STAGE_A = TC_BM * TC_BK * 2 * PARTS;
+  static constexpr int STAGE_B = (BN / CTAS) * TC_BK * 2 * PARTS;
   static constexpr int STAGE = STAGE_A + STAGE_B;
-  static constexpr int STAGES = CTAS == 2 ? (BN >= 192 ? 6 : 8) : ((BN == 256) ? 4 : (BN == 192 ? 4 : (BN == 128 ? 6 : 8)));
+  static constexpr int STAGES = TF32 ? 196608 / STAGE : CTAS == 2 ? (BN >= 192 ? 6 : 8) : ((BN == 256) ? 4 : (BN == 192 ? 4 : (BN == 128 ? 6 : 8)));
   static constexpr int EPI = 8 * 32 * 32 * 4;
   static constexpr int BYTES = STAGES * STAGE + EPI + 256 + 1024; /* + barriers + alignment slack */
 };
@@ -142,8 +144,8 @@ struct TcSmem {
 template <int BN, int CTAS, bool PROMOTE = false, bool TF32 = false, bool MN = false>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 pb200_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const TcArgs g) {
-  using S = TcSmem<BN, CTAS>;
-  static_assert(!PROMOTE || (CTAS == 1 && BN <= 128), "partial sums in registers: single CTAs, tiles up to 128 wide");
+  using S = TcSmem<BN, CTAS, TF32>;
+  static_assert(S::BYTES <= 227 * 1024 - 64, "shared memory");
   /* CTA pair: rank within the pair, the pair's index and count (tiles are handed out per pair) */
   const uint32_t rank = CTAS == 2 ? cluster_ctarank() : 0u;
   const int unit = blockIdx.x / CTAS, n_units = gridDim.x / CTAS;
@@ -204,12 +206,28 @@ pb200_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
             const uint32_t full0 = mapa_shared(bar_full + 8 * stage, 0);
             if (rank == 0) mbar_expect_tx(bar_full + 8 * stage, 2 * S::STAGE);
             const int ra = (mt * 2 + (int)rank) * TC_BM, rb = nt * BN + (int)rank * (BN / 2);
+            if constexpr (TF32) {
+              tma_load_3d_pair(sa, &map_a, full0, kb * bk, ra, bz);
+              tma_load_3d_pair(sa + S::STAGE_A / 2, &map_a, full0, kb * bk, ra, bz + g.nbatch);
+              tma_load_3d_pair(sb, &map_b, full0, kb * bk, rb, bz);
+              tma_load_3d_pair(sb + S::STAGE_B / 2, &map_b, full0, kb * bk, rb, bz + g.nbatch);
+              if (++stage == S::STAGES) { stage = 0; phase ^= 1u; }
+              continue;
+            }
             if (MN && g.a_mn) for (int i = 0; i < TC_BM / 64; i++) tma_load_3d_pair(sa + i * MN_BOX, &map_a, full0, ra + i * 64, kb * bk, bz);
             else tma_load_3d_pair(sa, &map_a, full0, kb * bk, ra, bz);
             if (MN && g.b_mn) for (int i = 0; i < BN / 2 / 64; i++) tma_load_3d_pair(sb + i * MN_BOX, &map_b, full0, rb + i * 64, kb * bk, bz);
             else tma_load_3d_pair(sb, &map_b, full0, kb * bk, rb, bz);
           } else {
             mbar_expect_tx(bar_full + 8 * stage, S::STAGE);
+            if constexpr (TF32) {
+              tma_load_3d(sa, &map_a, bar_full + 8 * stage, kb * bk, mt * TC_BM, bz);
+              tma_load_3d(sa + S::STAGE_A / 2, &map_a, bar_full + 8 * stage, kb * bk, mt * TC_BM, bz + g.nbatch);
+              tma_load_3d(sb, &map_b, bar_full + 8 * stage, kb * bk, nt * BN, bz);
+              tma_load_3d(sb + S::STAGE_B / 2, &map_b, bar_full + 8 * stage, kb * bk, nt * BN, bz + g.nbatch);
+              if (++stage == S::STAGES) { stage = 0; phase ^= 1u; }
+              continue;
+            }
             if (MN && g.a_mn) for (int i = 0; i < TC_BM / 64; i++) tma_load_3d(sa + i * MN_BOX, &map_a, bar_full + 8 * stage, mt * TC_BM + i * 64, kb * bk, bz);
             else tma_load_3d(sa, &map_a, bar_full + 8 * stage, kb * bk, mt * TC_BM, bz);
             if (MN && g.b_mn) for (int i = 0; i < BN / 64; i++) tma_load_3d(sb + i * MN_BOX, &map_b, bar_full + 8 * stage, nt * BN + i * 64, kb * bk, bz);
@@ -236,14 +254,23 @@ pb200_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
       auto issue_block = [&](uint32_t tmem_d, bool first) {
         const uint32_t sa = base + stage * S::STAGE, sb = sa + S::STAGE_A;
         const uint64_t da = a_mn ? make_smem_desc_mn(sa, MN_BOX) : make_smem_desc(sa), db = b_mn ? make_smem_desc_mn(sb, MN_BOX) : make_smem_desc(sb);
+        if constexpr (TF32) {
+          /* a.b = lo.hi + hi.lo + hi.hi, the small products first: the accumulation in tensor memory
+           * truncates, and truncates less while the sum is small */
+          constexpr uint64_t lo_a = S::STAGE_A / 32, lo_b = S::STAGE_B / 32;
 #pragma unroll
-        for (int k = 0; k < TC_BK / 16; k++) {
-          const uint32_t accum = (!first || k) ? 1u : 0u;
-          if constexpr (CTAS == 2) {
-            if constexpr (TF32) tc_mma_tf32_pair(tmem_d, da + k * ka, db + k * kb, idesc, accum);
-            else tc_mma_bf16_pair(tmem_d, da + k * ka, db + k * kb, idesc, accum);
-          } else {
-            if constexpr (TF32) tc_mma_tf32(tmem_d, da + k * ka, db + k * kb, idesc, accum);
+          for (int part = 0; part < 3; part++)
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+              const uint32_t accum = (!first || part || k) ? 1u : 0u;
+              const uint64_t pa = da + (part == 0 ? lo_a : 0) + k * 2, pb = db + (part == 1 ? lo_b : 0) + k * 2;
+              if constexpr (CTAS == 2) tc_mma_tf32_pair(tmem_d, pa, pb, idesc, accum); else tc_mma_tf32(tmem_d, pa, pb, idesc, accum);
+            }
+        } else {
+#pragma unroll
+          for (int k = 0; k < TC_BK / 16; k++) {
+            const uint32_t accum = (!first || k) ? 1u : 0u;
+            if constexpr (CTAS == 2) tc_mma_bf16_pair(tmem_d, da + k * ka, db + k * kb, idesc, accum);
             else tc_mma_bf16(tmem_d, da + k * ka, db + k * kb, idesc, accum);
           }
         }
@@ -281,7 +308,7 @@ pb200_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
               tc_fence_after_sync();
               issue_block(tmem_d, kblk == kb0);
             }
-            if (ok) tc_commit(bar_tfull + 8 * buf);
+            if (ok) { if constexpr (CTAS == 2) tc_commit_pair(bar_tfull + 8 * buf, 3); else tc_commit(bar_tfull + 8 * buf); }
           }
         }
       }
@@ -349,15 +376,22 @@ pb200_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
 #pragma unroll
           for (int ci = 0; ci < NCH; ci++) {
             if (colh + ci * 32 < g.N) {
-              uint32_t part[32];
-              tc_ld32(tb + ci * 32, part);
-              tc_wait_ld();
+              /* 16 columns at a time: a thread has 168 registers, 128 of them hold the sums of a 256-wide tile */
 #pragma unroll
-              for (int j = 0; j < 32; j++) acc[ci][j] += __uint_as_float(part[j]);
+              for (int h = 0; h < 2; h++) {
+                uint32_t part[16];
+                tc_ld16(tb + ci * 32 + h * 16, part);
+                tc_wait_ld();
+#pragma unroll
+                for (int j = 0; j < 16; j++) acc[ci][h * 16 + j] += __uint_as_float(part[j]);
+              }
             }
           }
           tc_fence_before_sync();
-          if (lane == 0) mbar_arrive(bar_tempty + 8 * buf);
+          if (lane == 0) {
+            if constexpr (CTAS == 2) mbar_arrive_cluster(mapa_shared(bar_tempty + 8 * buf, 0));
+            else mbar_arrive(bar_tempty + 8 * buf);
+          }
         }
         if (!ok) break;
       } else {
@@ -621,8 +655,8 @@ template <int BN, int CTAS, bool PROMOTE = false, bool TF32 = false, bool MN = f
 static int tc_configure() {
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(pb200_gemm_tc<BN, CTAS, PROMOTE, TF32, MN>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcSmem<BN, CTAS>::BYTES);
-    if (e != cudaSuccess) { pb_set_error("gemm: cannot reserve %d bytes of shared memory: %s", TcSmem<BN, CTAS>::BYTES, cudaGetErrorString(e)); return -1; }
+    cudaError_t e = cudaFuncSetAttribute(pb200_gemm_tc<BN, CTAS, PROMOTE, TF32, MN>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcSmem<BN, CTAS, TF32>::BYTES);
+    if (e != cudaSuccess) { pb_set_error("gemm: cannot reserve %d bytes of shared memory: %s", TcSmem<BN, CTAS, TF32>::BYTES, cudaGetErrorString(e)); return -1; }
     configured = true;
   }
   return 0;
@@ -651,11 +685,11 @@ static int tc_launch(const CUtensorMap &ma, const CUtensorMap &mb, TcArgs &g, lo
   const int grid = (int)(tiles < units ? tiles : units) * CTAS;
   cudaError_t e;
   if (CTAS == 1) {
-    pb200_gemm_tc<BN, CTAS, PROMOTE, TF32, MN><<<grid, TC_THREADS, TcSmem<BN, CTAS>::BYTES, stream>>>(ma, mb, g);
+    pb200_gemm_tc<BN, CTAS, PROMOTE, TF32, MN><<<grid, TC_THREADS, TcSmem<BN, CTAS, TF32>::BYTES, stream>>>(ma, mb, g);
     e = cudaGetLastError();
   } else {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid); cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = TcSmem<BN, CTAS>::BYTES; cfg.stream = stream;
+    cfg.gridDim = dim3((unsigned)grid); cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = TcSmem<BN, CTAS, TF32>::BYTES; cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = CTAS; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
@@ -715,10 +749,13 @@ static const void *tc_operand(PbGemmProgram &p, PbTcOperand &cache, const void *
 
 /* ── fp32 contractions on the tensor cores: three tf32 products ─────────
  * a = hi + lo with hi = tf32(a), lo = tf32(a - hi) carries 22 bits of a's
- * mantissa; a.b ~ hi.hi + hi.lo + lo.hi leaves out terms of relative size
- * 2^-22.  The three products are one contraction over a k axis three times as
- * long: A' = [hi | hi | lo], B' = [hi | lo | hi], each segment Kp = K rounded up
- * to 4 elements (16-byte rows) and zero-filled past K.  Accumulation is fp32 in
+ * mantissa; a.b ~ lo.hi + hi.lo + hi.hi leaves out terms of relative size
+ * 2^-22.  An operand is split once into two K-major matrices, its hi parts and
+ * its lo parts (rows of Kp = K rounded up to 4 floats: 16-byte rows); a stage of
+ * the kernel holds both parts of both tiles and feeds all three products.
+ * (One contraction over [hi | hi | lo] and [hi | lo | hi] moved 128 x 128 tiles at
+ * 128 bytes per clock and SM from L2 and was bound by that: 8192 x 2304 x 768 took
+ * 244 us with the splits, 768 x 3072 x 4096 238.)  Accumulation is fp32 in
  * TMEM, which truncates: summed over the whole k axis there, the error against
  * a float64 product is about 1e-8 * K of the result's rms (a CPU float32 sum:
  * 2e-7 to 4e-7).  The PROMOTE kernels therefore hand the partial sum of every
@@ -730,97 +767,84 @@ __device__ __forceinline__ float tf32_rna(float a) {
   return __uint_as_float(u);
 }
 
-struct SplitSrc {                      /* the source as [batch axes][rows][k], k contiguous */
-  const float *src; long long pitch; long long rows;
-  int nb; int bext[4]; long long bstr[4];
-};
-
-/* one value into its three segments: x0 goes to [0, Kp), x1 to [Kp, 2Kp), x2 to [2Kp, 3Kp) */
-__device__ __forceinline__ void split_one(float a, int is_b, float &x0, float &x1, float &x2) {
+__device__ __forceinline__ void split_one(float a, float &hi, float &lo) {
   if (!(fabsf(a) <= 3.4028235e38f)) {
-    /* an infinity or a NaN meets only the other operand's hi part, once: inf * b keeps b's sign
-     * (and inf * 0 is NaN) as in the plain product, instead of meeting lo parts of either sign */
-    x0 = a; x1 = 0.0f; x2 = 0.0f;
+    /* an infinity or a NaN is the lo part beside a hi part of its sign: it then meets the other operand's hi
+     * part once (inf * b keeps b's sign, inf * 0 is NaN) and never a lo part, which has either sign; two
+     * infinities meet as 1 * inf + inf * 1 */
+    hi = copysignf(1.0f, a); lo = a;
     return;
   }
-  float hi = tf32_rna(a);
+  hi = tf32_rna(a);
   if (!(fabsf(hi) <= 3.4028235e38f)) hi = __uint_as_float(__float_as_uint(a) & 0xffffe000u);   /* rounding overflowed: truncate */
-  const float lo = tf32_rna(a - hi);
-  x0 = hi; x1 = is_b ? lo : hi; x2 = is_b ? hi : lo;
+  lo = tf32_rna(a - hi);
 }
 
-__global__ void __launch_bounds__(256) pb200_split_tf32x3(const SplitSrc in, float *__restrict__ dst,
-                                                          long long total, int K, int Kp, int is_b) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long row = i / Kp; const int k = (int)(i % Kp);
-    long long bz = row / in.rows, so = (row % in.rows) * in.pitch;
-    for (int d = 0; d < in.nb; d++) { so += (bz % in.bext[d]) * in.bstr[d]; bz /= in.bext[d]; }
-    const float a = k < K ? in.src[so + k] : 0.0f;
-    float *o = dst + row * 3 * Kp;
-    split_one(a, is_b, o[k], o[Kp + k], o[2 * Kp + k]);
-  }
-}
-
-/* The same with four consecutive k per thread: one 128-bit load, three 128-bit stores.  Needs rows of the
- * source that start on 16-byte boundaries (Kp is a multiple of 4, so the destination's always do). */
-__global__ void __launch_bounds__(256) pb200_split_tf32x3_v4(const SplitSrc in, float *__restrict__ dst,
-                                                             long long total4, int K, int Kp, int is_b) {
-  const int kq = Kp >> 2;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total4; i += (long long)gridDim.x * blockDim.x) {
-    const long long row = i / kq; const int k = (int)(i % kq) << 2;
-    long long bz = row / in.rows, so = (row % in.rows) * in.pitch;
-    for (int d = 0; d < in.nb; d++) { so += (bz % in.bext[d]) * in.bstr[d]; bz /= in.bext[d]; }
-    float4 a;
-    if (k + 3 < K) a = *reinterpret_cast<const float4 *>(in.src + so + k);
-    else {
-      a.x = k < K ? in.src[so + k] : 0.0f; a.y = k + 1 < K ? in.src[so + k + 1] : 0.0f;
-      a.z = k + 2 < K ? in.src[so + k + 2] : 0.0f; a.w = 0.0f;
-    }
-    float4 x0, x1, x2;
-    split_one(a.x, is_b, x0.x, x1.x, x2.x); split_one(a.y, is_b, x0.y, x1.y, x2.y);
-    split_one(a.z, is_b, x0.z, x1.z, x2.z); split_one(a.w, is_b, x0.w, x1.w, x2.w);
-    float *o = dst + row * 3 * Kp + k;
-    *reinterpret_cast<float4 *>(o) = x0;
-    *reinterpret_cast<float4 *>(o + Kp) = x1;
-    *reinterpret_cast<float4 *>(o + 2 * Kp) = x2;
-  }
-}
-
-/* An operand stored with its row axis contiguous and k strided (a weight gradient reads the
- * activations transposed): 32 x 32 tiles through shared memory, read along the rows, written along k
- * in the split form.  dst row of (batch z, r) is z * R + r; k in [K, Kp) is zero-filled. */
-struct SplitTrArgs {
-  const float *src; float *dst;
-  int R, K, Kp; long long s_k;
+/* One operand into its two parts.  The source is [batch axes][R][K] with k contiguous (kfast) or the row
+ * axis contiguous; the result is rows z * R + r of Kp floats, hi parts at dst, lo parts at dst + plane.  A
+ * block takes 64 rows x 64 k: 128-bit loads along the contiguous axis where the source allows (vec), through
+ * shared memory if that is the row axis, 128-bit stores along k.  Bound by memory: 4 bytes read, 8 written per element. */
+struct SplitArgs {
+  const float *src; float *dst; long long plane;
+  int R, K, Kp, vec;
+  long long pitch;                                 /* between rows (kfast) or between k */
   int naxes; int ext[6]; long long sstride[6];     /* the other axes of the source, fastest first */
-  int is_b;
+  int tr, tk;                                      /* 64-wide tiles along the rows and along k */
 };
 
-__global__ void __launch_bounds__(256) pb200_split_tf32x3_tr(const SplitTrArgs a) {
-  __shared__ float tile[32][33];
-  long long rem = blockIdx.z, o = 0;
+template <bool KFAST>
+__global__ void __launch_bounds__(256) pb200_split_tf32(const SplitArgs a) {
+  __shared__ float tile[KFAST ? 1 : 64][65];       /* [k][row] */
+  const int t = blockIdx.x % (a.tr * a.tk), z = blockIdx.x / (a.tr * a.tk);
+  const int r0 = (t / a.tk) * 64, k0 = (t % a.tk) * 64;
+  long long rem = z, o = 0;
   for (int d = 0; d < a.naxes; d++) { const long long x = rem % a.ext[d]; rem /= a.ext[d]; o += x * a.sstride[d]; }
-  const int r0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  for (int j = ty; j < 32; j += 8) {
-    const int k = k0 + j, r = r0 + tx;
-    tile[j][tx] = (k < a.K && r < a.R) ? a.src[o + (long long)k * a.s_k + r] : 0.0f;
+  const float *src = a.src + o;
+  const int q = (threadIdx.x & 15) * 4, line = threadIdx.x >> 4;
+  float4 v[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    /* line: row (kfast) or k; q: position along the contiguous axis */
+    const int l = (KFAST ? r0 : k0) + line + i * 16, c = (KFAST ? k0 : r0) + q;
+    const int nl = KFAST ? a.R : a.K, nc = KFAST ? a.K : a.R;
+    const float *p = src + (long long)l * a.pitch + c;
+    if (l < nl && a.vec && c + 3 < nc) v[i] = __ldg(reinterpret_cast<const float4 *>(p));
+    else {
+      v[i].x = l < nl && c < nc ? p[0] : 0.0f; v[i].y = l < nl && c + 1 < nc ? p[1] : 0.0f;
+      v[i].z = l < nl && c + 2 < nc ? p[2] : 0.0f; v[i].w = l < nl && c + 3 < nc ? p[3] : 0.0f;
+    }
   }
-  __syncthreads();
-  for (int j = ty; j < 32; j += 8) {
-    const int r = r0 + j, k = k0 + tx;
+  if (!KFAST) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      float *s = &tile[line + i * 16][q];
+      s[0] = v[i].x; s[1] = v[i].y; s[2] = v[i].z; s[3] = v[i].w;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int r = line + i * 16;
+      v[i] = make_float4(tile[q][r], tile[q + 1][r], tile[q + 2][r], tile[q + 3][r]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int r = r0 + line + i * 16, k = k0 + q;
     if (r < a.R && k < a.Kp) {
-      float *d = a.dst + ((long long)blockIdx.z * a.R + r) * 3 * a.Kp;
-      split_one(tile[tx][j], a.is_b, d[k], d[a.Kp + k], d[2 * a.Kp + k]);
+      float4 hi, lo;
+      split_one(v[i].x, hi.x, lo.x); split_one(v[i].y, hi.y, lo.y); split_one(v[i].z, hi.z, lo.z); split_one(v[i].w, hi.w, lo.w);
+      float *d = a.dst + ((long long)z * a.R + r) * a.Kp + k;
+      *reinterpret_cast<float4 *>(d) = hi;
+      *reinterpret_cast<float4 *>(d + a.plane) = lo;
     }
   }
 }
 
-/* [nbatch][rows][3 * Kp] float32 copy of A or B in the split form; cached like the bf16 copies. */
+/* The two parts of A or B, [2][nbatch][rows][Kp] float32; cached like the bf16 copies. */
 static const void *tc_operand_x3(PbGemmProgram &p, PbTcOperand &cache, const void *src_buf, long long off, bool is_a,
                                  long long rows, long long Kp, cudaStream_t stream, void **scratch) {
   *scratch = nullptr;
-  const size_t bytes = (size_t)(p.nbatch * rows * 3 * Kp) * 4;
+  const size_t bytes = (size_t)(p.nbatch * rows * 2 * Kp) * 4;
   const uint64_t ver = pb_buffer_version(src_buf);
   if (cache.data && cache.src == src_buf && cache.version == ver && cache.bytes == bytes && ver != 0) return cache.data;
   const bool transient = cache.misses >= 2 || ver == 0;
@@ -837,62 +861,40 @@ static const void *tc_operand_x3(PbGemmProgram &p, PbTcOperand &cache, const voi
     dst = cache.data;
     cache.src = src_buf; cache.version = ver; cache.misses++;
   }
-  /* an operand that already is a K-major matrix (an activation as the model stores it) is split
-   * where it lies; anything else is gathered into a dense [rows][Kp] copy first */
+  /* an operand whose strides nest and whose k or row axis is contiguous (an activation as the model stores it;
+   * a weight; the activations a weight gradient reads transposed, whose token axes nest into one k axis) is
+   * split where it lies; anything else is gathered into a dense [rows][Kp] copy first */
+  auto sel = [&](const PbGemmAxis &x) { return is_a ? x.sa : x.sb; };
   const bool direct = is_a ? p.a_direct : p.b_direct;
   const long long sk = is_a ? p.a_sk : p.b_sk, srow = is_a ? p.a_sm : p.b_sn;
-  bool in_place = direct && (sk == 1 || p.K == 1) && srow >= 0 && p.b_ax.size() <= 4;
-  for (auto &b : p.b_ax) if ((is_a ? b.sa : b.sb) < 0) in_place = false;
+  const char *e = getenv("POLY_B200_SPLIT_TR");            /* "0": gather an operand with contiguous rows first (measurements) */
+  const bool kfast = sk == 1 || p.K == 1;
+  bool in_place = direct && p.b_ax.size() <= 6 && rows <= 2147483647LL - 64 &&
+                  (kfast ? srow >= 0 : (srow == 1 && sk > 1 && rows > 1 && !(e && e[0] == '0')));
+  long long nz = 1;
+  for (auto &b : p.b_ax) { if (sel(b) < 0) in_place = false; nz *= b.ext; }
   void *dense = nullptr;
   bool ok = true;
-  SplitSrc in{};
-  in.rows = rows;
+  SplitArgs a{};
+  a.dst = (float *)dst; a.plane = p.nbatch * rows * Kp; a.K = (int)p.K; a.Kp = (int)Kp;
   if (in_place) {
-    in.src = (const float *)src_buf + off; in.pitch = rows > 1 ? srow : 0;
-    in.nb = (int)p.b_ax.size();
-    for (int i = 0; i < in.nb; i++) { in.bext[i] = (int)p.b_ax[i].ext; in.bstr[i] = is_a ? p.b_ax[i].sa : p.b_ax[i].sb; }
+    a.src = (const float *)src_buf + off; a.R = (int)rows;
+    a.pitch = kfast ? (rows > 1 ? srow : 0) : sk;
+    for (auto &b : p.b_ax) { a.ext[a.naxes] = (int)b.ext; a.sstride[a.naxes++] = sel(b); }
   } else {
-    /* a strided matrix per batch entry with its rows contiguous and k strided (a weight gradient reads the
-     * activations transposed; the token axes (batch, position) nest into one k axis): transposed and split
-     * in one pass */
-    auto sel = [&](const PbGemmAxis &x) { return is_a ? x.sa : x.sb; };
-    const char *e = getenv("POLY_B200_SPLIT_TR");
-    if (!(e && e[0] == '0') && direct && srow == 1 && sk > 1 && rows > 1 && p.b_ax.size() <= 6 && rows <= 2147483647LL) {
-      SplitTrArgs t{};
-      t.src = (const float *)src_buf + off; t.dst = (float *)dst;
-      t.R = (int)rows; t.K = (int)p.K; t.Kp = (int)Kp; t.s_k = sk; t.is_b = is_a ? 0 : 1;
-      long long nz = 1;
-      bool fits = true;
-      for (size_t i = 0; i < p.b_ax.size(); i++) {
-        if (sel(p.b_ax[i]) < 0) fits = false;
-        t.ext[t.naxes] = (int)p.b_ax[i].ext; t.sstride[t.naxes++] = sel(p.b_ax[i]); nz *= p.b_ax[i].ext;
-      }
-      if (nz > 65535 || (Kp + 31) / 32 > 65535) fits = false;
-      if (fits) {
-        dim3 grid((unsigned)((t.R + 31) / 32), (unsigned)((Kp + 31) / 32), (unsigned)nz);
-        pb200_split_tf32x3_tr<<<grid, 256, 0, stream>>>(t);
-        ok = cudaGetLastError() == cudaSuccess;
-        p.launches++;
-        if (!ok) {
-          if (*scratch) { pb_scratch_free(*scratch); *scratch = nullptr; }
-          else cache.version = 0;
-          return nullptr;
-        }
-        return dst;
-      }
-    }
-    dense = pb_scratch_alloc((size_t)(p.nbatch * rows * Kp) * 4);
+    if (p.nbatch * rows > 2147483647LL - 64) ok = false;
+    dense = ok ? pb_scratch_alloc((size_t)(p.nbatch * rows * Kp) * 4) : nullptr;
     ok = dense != nullptr && p.pack_into(dense, src_buf, off, is_a, PB_F32, PB_F32, Kp, stream) == 0;
-    in.src = (const float *)dense; in.pitch = Kp; in.rows = p.nbatch * rows; in.nb = 0;
+    a.src = (const float *)dense; a.R = (int)(p.nbatch * rows); a.pitch = Kp; nz = 1;
   }
+  a.vec = (reinterpret_cast<uintptr_t>(a.src) & 15) == 0 && a.pitch % 4 == 0;
+  for (int i = 0; i < a.naxes; i++) if (a.sstride[i] % 4) a.vec = 0;
+  a.tr = (a.R + 63) / 64; a.tk = ((int)Kp + 63) / 64;
+  const long long blocks = (long long)a.tr * a.tk * nz;
+  if (blocks > 2147483647LL) { pb_set_error("gemm: operand too large to split"); ok = false; }
   if (ok) {
-    const long long total = p.nbatch * rows * Kp;
-    bool v4 = (reinterpret_cast<uintptr_t>(in.src) & 15) == 0 && in.pitch % 4 == 0;
-    for (int i = 0; i < in.nb; i++) if (in.bstr[i] % 4) v4 = false;
-    long long blocks = ((v4 ? total / 4 : total) + 255) / 256;
-    if (blocks > 148LL * 32) blocks = 148LL * 32;
-    if (v4) pb200_split_tf32x3_v4<<<(unsigned)blocks, 256, 0, stream>>>(in, (float *)dst, total / 4, (int)p.K, (int)Kp, is_a ? 0 : 1);
-    else pb200_split_tf32x3<<<(unsigned)blocks, 256, 0, stream>>>(in, (float *)dst, total, (int)p.K, (int)Kp, is_a ? 0 : 1);
+    if (in_place && !kfast) pb200_split_tf32<false><<<(unsigned)blocks, 256, 0, stream>>>(a);
+    else pb200_split_tf32<true><<<(unsigned)blocks, 256, 0, stream>>>(a);
     ok = cudaGetLastError() == cudaSuccess;
     p.launches++;
   }
@@ -970,11 +972,11 @@ int pb_gemm_tc_run(PbGemmProgram &p, void *const *bufs, cudaStream_t stream, int
   void *scr_a = nullptr, *scr_b = nullptr;
   TcView va, vb;
   if (fp32x3) {
-    if (p.dtype != PB_F32 || p.a_bf16 || p.c_bf16 || 3 * Kp > 2147483647LL) return PB_TC_UNSUPPORTED;
+    if (p.dtype != PB_F32 || p.a_bf16 || p.c_bf16 || 2 * p.nbatch > 2147483647LL) return PB_TC_UNSUPPORTED;
     va.ptr = tc_operand_x3(p, p.tc_a, bufs[p.p_a], p.off_a, true, p.M, Kp, stream, &scr_a);
-    va.pitch = 3 * Kp; va.bpitch = p.M * 3 * Kp;
+    va.pitch = Kp; va.bpitch = p.M * Kp;
     vb.ptr = va.ptr ? tc_operand_x3(p, p.tc_b, bufs[p.p_b], p.off_b, false, p.N, Kp, stream, &scr_b) : nullptr;
-    vb.pitch = 3 * Kp; vb.bpitch = p.N * 3 * Kp;
+    vb.pitch = Kp; vb.bpitch = p.N * Kp;
   } else if (!tc_in_place(p, bufs[p.p_a], p.off_a, true, &va)) {
     if (p.a_bf16) { pb_set_error("gemm: bfloat16 A operand is not addressable in place (alignment)"); return -1; }
     if (!tc_in_place_mn(p, bufs[p.p_a], p.off_a, true, &va)) {
@@ -991,7 +993,7 @@ int pb_gemm_tc_run(PbGemmProgram &p, void *const *bufs, cudaStream_t stream, int
   TcArgs g{};
   long long rowsA = p.M, rowsB = p.N;
   if (swap) { std::swap(va, vb); std::swap(rowsA, rowsB); }
-  g.M = (int)rowsA; g.N = (int)rowsB; g.K = fp32x3 ? (int)(3 * Kp) : (int)p.K;
+  g.M = (int)rowsA; g.N = (int)rowsB; g.K = (int)p.K; g.nbatch = (int)p.nbatch;
   g.C = (float *)bufs[p.p_c] + p.off_c;
   g.c_sm = swap ? p.c_sn : p.c_sm;
   g.has_x = p.has_x ? 1 : 0; g.relu = p.relu ? 1 : 0;
@@ -1034,7 +1036,7 @@ int pb_gemm_tc_run(PbGemmProgram &p, void *const *bufs, cudaStream_t stream, int
    * operand bytes per flop) */
   int BN = 256;
   double best_cost = 0;
-  const double k_model = fp32x3 ? 2.0 * g.K : (double)g.K;      /* in 2-byte elements: a tf32 tile row holds half as many */
+  const double k_model = fp32x3 ? 6.0 * g.K : (double)g.K;      /* in 2-byte elements: three products, and a tf32 tile row holds half as many */
   {
     static const int widths[4] = {64, 128, 192, 256};
     double best = -1;
@@ -1056,7 +1058,8 @@ int pb_gemm_tc_run(PbGemmProgram &p, void *const *bufs, cudaStream_t stream, int
    * 8192 x 3072 x 1024 915 -> 999, 8192 x 2304 x 768 802 -> 765).  In the time model a pair's mainloop costs 0.85 of two single
    * tiles'.  POLY_B200_TC_CTAS=1|2 forces the choice (2 implies the 256-wide tile). */
   int ctas = 1;
-  if (!promote && g.M > TC_BM && g.N > 128) {
+  /* (float32: 256 x 256 pairs against single CTAs 128 wide, 8192 x 2304 x 768: 160 and 188 us; 256 x 128 pairs were slower than both) */
+  if (g.M > TC_BM && g.N > 128) {
     const long long pair_tiles = ((g.M + 2 * TC_BM - 1) / (2 * TC_BM)) * ((g.N + 255) / 256) * p.nbatch;
     const double pair_cost = (double)((pair_tiles + 73) / 74) * (0.85 * k_model * 256 + 94000.0);
     if (k_model >= 1024 && pair_tiles >= 74 && pair_cost <= best_cost && !getenv("POLY_B200_TC_BN")) { ctas = 2; BN = 256; }
@@ -1066,21 +1069,23 @@ int pb_gemm_tc_run(PbGemmProgram &p, void *const *bufs, cudaStream_t stream, int
   }
   CUtensorMap ma, mb;
   g.a_mn = va.mn; g.b_mn = vb.mn;
-  int rc = va.mn ? make_map(&ma, va.ptr, rowsA, g.K, p.nbatch, va.pitch, va.bpitch, TC_BK, g.ab_fmt)
-                 : make_map(&ma, va.ptr, g.K, rowsA, p.nbatch, va.pitch, va.bpitch, TC_BM, g.ab_fmt);
-  if (rc == 0) rc = vb.mn ? make_map(&mb, vb.ptr, rowsB, g.K, p.nbatch, vb.pitch, vb.bpitch, TC_BK, g.ab_fmt)
-                          : make_map(&mb, vb.ptr, g.K, rowsB, p.nbatch, vb.pitch, vb.bpitch, BN / ctas, g.ab_fmt);
+  const long long n_maps = fp32x3 ? 2 * p.nbatch : p.nbatch;
+  int rc = va.mn ? make_map(&ma, va.ptr, rowsA, g.K, n_maps, va.pitch, va.bpitch, TC_BK, g.ab_fmt)
+                 : make_map(&ma, va.ptr, g.K, rowsA, n_maps, va.pitch, va.bpitch, TC_BM, g.ab_fmt);
+  if (rc == 0) rc = vb.mn ? make_map(&mb, vb.ptr, rowsB, g.K, n_maps, vb.pitch, vb.bpitch, TC_BK, g.ab_fmt)
+                          : make_map(&mb, vb.ptr, g.K, rowsB, n_maps, vb.pitch, vb.bpitch, BN / ctas, g.ab_fmt);
   if (rc != 0) { pb_scratch_free(scr_a); pb_scratch_free(scr_b); return -1; }
   pb_tc_mark_used();
   pb_tc_configure_backoff();
   if (promote) {
-    /* eight 128-byte k-blocks (32 instructions, 256 elements of the tripled k axis) per partial sum:
-     * measured on GPT-2 124M fp32, 2 blocks cost 58.9 ms per step, 4: 45.2, 8: 43.7, 16: 43.1 (no
-     * promotion: 42.5), and at 16 the error against a float64 product starts to show;
-     * POLY_B200_TC_KCHUNK overrides (measurements) */
+    /* two 32-float k-blocks (24 instructions) per partial sum.  Error against a float64 product (rms, N(0, 1)
+     * operands, K 768 to 16384) and time of 8192 x 2304 x 768: 1 block 1.6e-7 to 4.3e-7, 190 us; 2 blocks 3.7e-7 to
+     * 4.7e-7, 157 us; 4 blocks 8.2e-7 to 8.5e-7, 149 us (256 elements of one 3K axis, as it was: 6.4e-7 to
+     * 7.1e-7, 244 us); POLY_B200_TC_KCHUNK overrides (measurements) */
     const char *kc = getenv("POLY_B200_TC_KCHUNK");
-    g.kchunk = kc && atoi(kc) > 0 ? atoi(kc) : 8;
-    rc = BN == 128 ? tc_launch<128, 1, true, true>(ma, mb, g, p.nbatch, stream) : tc_launch<64, 1, true, true>(ma, mb, g, p.nbatch, stream);
+    g.kchunk = kc && atoi(kc) > 0 ? atoi(kc) : 2;
+    if (ctas == 2) rc = tc_launch<256, 2, true, true>(ma, mb, g, p.nbatch, stream);
+    else rc = BN == 128 ? tc_launch<128, 1, true, true>(ma, mb, g, p.nbatch, stream) : tc_launch<64, 1, true, true>(ma, mb, g, p.nbatch, stream);
   } else if (fp32x3) {
     if (ctas == 2) rc = tc_launch<256, 2, false, true>(ma, mb, g, p.nbatch, stream);
     else if (BN == 256) rc = tc_launch<256, 1, false, true>(ma, mb, g, p.nbatch, stream);

@@ -57,3 +57,39 @@ def run_bf16(kernels, m, n, k, a_kfast, b_kfast, pad):  # noqa: F811
     assert kernels.c.poly_b200_gemm(m, n, k, kernels.put(ma), a_sm, a_sk, kernels.put(mb), b_sk, b_sn, c, n, kernels.put(bias), 0, 1) == 0, kernels.error()
     want = a.astype(np.float64) @ b.T.astype(np.float64) + bias
     assert_close(kernels.get(c, (m, n)), want, 1e-4, f'bf16 {m} {n} {k}')
+
+
+F32_SIZES = [(128, 64, 64), (197, 200, 768), (130, 257, 100), (64, 264, 1032), (300, 136, 17), (520, 1030, 333), (2312, 2184, 200)]
+
+
+@pytest.mark.parametrize('pad', [0, 3])
+@pytest.mark.parametrize('a_kfast,b_kfast', [(True, False), (True, True), (False, False), (False, True)])
+@pytest.mark.parametrize('m,n,k', F32_SIZES, ids=str)
+def test_f32_operands_on_the_tensor_cores(kernels, monkeypatch, m, n, k, a_kfast, b_kfast, pad):  # noqa: F811
+    """Every form of the three-product route (single CTAs, pairs, both orders of each operand): float32 accuracy."""
+    monkeypatch.setenv('POLY_B200_FP32', 'tcp')
+    rng = np.random.default_rng([m, n, k, pad])
+    a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
+    bias = rng.standard_normal(n).astype(np.float32)
+    ma, (a_sm, a_sk) = stored(a, a_kfast, pad, rng, lambda x: x)
+    mb, (b_sn, b_sk) = stored(b, b_kfast, pad, rng, lambda x: x)
+    c = kernels.put(np.zeros((m, n), np.float32))
+    assert kernels.c.poly_b200_gemm(m, n, k, kernels.put(ma), a_sm, a_sk, kernels.put(mb), b_sk, b_sn, c, n, kernels.put(bias), 0, 0) == 0, kernels.error()
+    want = a.astype(np.float64) @ b.T.astype(np.float64) + bias
+    assert_close(kernels.get(c, (m, n)), want, 1e-5, f'f32 {m} {n} {k}')
+
+
+def test_f32_infinities_on_the_tensor_cores(kernels, monkeypatch):  # noqa: F811
+    """An infinity meets finite values of either sign, zeros (NaN), another infinity, a NaN."""
+    monkeypatch.setenv('POLY_B200_FP32', 'tcp')
+    m, n, k = 128, 64, 32
+    rng = np.random.default_rng(1)
+    a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((k, n)).astype(np.float32)
+    a[3, 5], a[7, 1], a[9, 2], a[11, 30] = np.inf, -np.inf, np.nan, 3.4e38
+    b[5, 4], b[5, 6], b[1, 8], b[8, 9] = 0.0, np.inf, -np.inf, -np.inf
+    c = kernels.put(np.zeros((m, n), np.float32))
+    assert kernels.c.poly_b200_gemm(m, n, k, kernels.put(a), k, 1, kernels.put(b), n, 1, c, n, None, 0, 0) == 0, kernels.error()
+    with np.errstate(all='ignore'):
+        want = (a[:, :, None].astype(np.float64) * b.astype(np.float64)).sum(1)
+    got, rows = kernels.get(c, (m, n)), np.arange(m) != 11         # a product near the largest float32 may round to infinity or not
+    assert_close(got[rows], want[rows], 1e-5, 'infinities')
