@@ -93,3 +93,16 @@ def test_f32_infinities_on_the_tensor_cores(kernels, monkeypatch):  # noqa: F811
         want = (a[:, :, None].astype(np.float64) * b.astype(np.float64)).sum(1)
     got, rows = kernels.get(c, (m, n)), np.arange(m) != 11         # a product near the largest float32 may round to infinity or not
     assert_close(got[rows], want[rows], 1e-5, 'infinities')
+
+
+@pytest.mark.parametrize('relu', [0, 1])
+@pytest.mark.parametrize('m,n,k', [(160, 257, 64), (31, 1001, 128), (2620, 51237, 16)], ids=str)
+def test_rows_of_float32_off_the_16_byte_grid(kernels, m, n, k, relu):  # noqa: F811
+    """Whole and ragged groups of 32 rows; the largest result (537 MB) is written with streaming stores."""
+    rng = np.random.default_rng([m, n])
+    a, b = bf16(rng.standard_normal((m, k))), bf16(rng.standard_normal((n, k)))
+    c = kernels.put(np.zeros((m, n), np.float32))
+    assert kernels.c.poly_b200_gemm(m, n, k, kernels.put(bits(a)), k, 1, kernels.put(bits(b)), 1, k, c, n, None, relu, 1) == 0, kernels.error()
+    got, want = kernels.get(c, (m, n)), a @ b.T
+    for r in range(0, m, 500):
+        assert_close(got[r:r + 500], np.maximum(want[r:r + 500], 0) if relu else want[r:r + 500], 1e-4, f'{m} {n} {k} from row {r}')
