@@ -339,14 +339,45 @@ static SgemmFn pick_vec(bool va, bool vb) {
   return pb200_sgemm<AK, BKm, false, false>;
 }
 
-/* Small problems: a 128 x 128 tiling would leave most SMs idle (the 256 x 784 x 512 and
- * 256 x 512 x 10 layers of an MLP are 8 and 2 such tiles).  32 x 32 tiles, 256 threads,
- * 2 x 2 results per thread, any strides; same accumulation as the large kernel
- * (k ascending, one fused multiply-add per product). */
-#define SB 32
-__global__ void __launch_bounds__(256) pb200_sgemm_small(const SgemmArgs g) {
-  __shared__ float As[2][SB][SB + 1];      /* [k][m] */
-  __shared__ float Bs[2][SB][SB + 1];      /* [k][n] */
+/* Small problems: 128 x 128 tiles would leave most SMs idle (the 256 x 784 x 512 and 256 x 512 x 10 layers of an
+ * MLP are 8 and 2 of them), so 64 x 64 tiles, and the k axis of a tile split twice: between the 2, 4 or 8 CTAs of a
+ * cluster, and between the four 64-thread groups of a CTA, which take every fourth quad of k.  A thread then still
+ * has 8 x 8 results (16 128-bit shared-memory loads per 256 multiply-adds; with 2 x 2 results shared memory was the
+ * bound), and four k slabs of 32 are in flight (cp.async, zero-filled past every edge).  Partial sums
+ * are added in a fixed order: groups in shared memory, then the CTAs of a cluster over distributed shared memory.
+ * 32 x 32 tiles with 2 x 2 results and one slab in flight: 256 x 512 x 784 28.7 us, 256 x 10 x 512 19.1 us;
+ * 18.1 and 10.2 like this. */
+#define SB 64
+#define SK 32
+#define S_STAGES 4
+#define S_OPERAND (SB * (SK + 4))                /* floats of one staged operand; [k][row] needs SK * (SB + 4), less */
+#define S_PITCH (SB + 8)                         /* of the partial sums, which reuse the stages */
+#define S_SMEM (S_STAGES * 2 * S_OPERAND * 4)
+static_assert(4 * SB * S_PITCH * 4 <= S_SMEM, "partial sums of four groups fit the stages");
+
+__device__ __forceinline__ void cp_async(uint32_t dst, const float *src, int bytes, bool wide) {
+  if (wide) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+/* 64 rows x 32 k of an operand: [row][k] where k is contiguous in memory, else [k][row] */
+template <bool KFAST>
+__device__ __forceinline__ void stage_operand(uint32_t dst, const float *base, long long s_row, long long s_k, int row0, int rows,
+                                              int k0, int kend, bool wide) {
+  const int per = wide ? 4 : 1, n = SB * SK / per;
+  for (int c = threadIdx.x; c < n; c += 256) {
+    const int e = c * per;
+    const int k = KFAST ? e % SK : e / SB, r = KFAST ? e / SK : e % SB;
+    const int left = KFAST ? (row0 + r < rows ? kend - k0 - k : 0) : (k0 + k < kend ? rows - row0 - r : 0);
+    const int bytes = 4 * max(0, min(per, left));
+    const float *src = bytes ? base + (long long)(row0 + r) * s_row + (long long)(k0 + k) * s_k : base;
+    cp_async(dst + 4 * (KFAST ? r * (SK + 4) + k : k * (SB + 4) + r), src, bytes, wide);
+  }
+}
+
+template <bool AK, bool BKm>
+__global__ void __launch_bounds__(256, 1) pb200_sgemm_small(const SgemmArgs g, const int n_split, const bool wide_a, const bool wide_b) {
+  extern __shared__ __align__(16) float sm[];
   long long oa = 0, ob = 0, oc = 0, ox = 0;
   {
     int rem = blockIdx.z;
@@ -357,91 +388,152 @@ __global__ void __launch_bounds__(256) pb200_sgemm_small(const SgemmArgs g) {
   }
   const float *__restrict__ A = g.A + oa;
   const float *__restrict__ B = g.B + ob;
-  const int m0 = blockIdx.y * SB, n0 = blockIdx.x * SB;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  /* element e of a 32 x 32 tile: consecutive threads along the operand's contiguous axis */
-  const bool a_kfast = g.a_sk == 1, b_kfast = g.b_sk == 1 && g.b_sn != 1;
-  float ra[4], rb[4];
-  auto fetch = [&](int k0) {
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int e = tid + i * 256;
-      const int ka = a_kfast ? (e & 31) : (e >> 5), ma = a_kfast ? (e >> 5) : (e & 31);
-      const int kb = b_kfast ? (e & 31) : (e >> 5), nb = b_kfast ? (e >> 5) : (e & 31);
-      ra[i] = (m0 + ma < g.M && k0 + ka < g.K) ? A[(long long)(m0 + ma) * g.a_sm + (long long)(k0 + ka) * g.a_sk] : 0.0f;
-      rb[i] = (n0 + nb < g.N && k0 + kb < g.K) ? B[(long long)(k0 + kb) * g.b_sk + (long long)(n0 + nb) * g.b_sn] : 0.0f;
+  const int rank = blockIdx.x % n_split;                     /* the cluster's CTAs are neighbours along x */
+  const int m0 = blockIdx.y * SB, n0 = (blockIdx.x / n_split) * SB;
+  const int group = threadIdx.x >> 6, tx = threadIdx.x & 7, ty = (threadIdx.x >> 3) & 7;
+  /* k-contiguous tiles are read a quad of k at a time, rows eight apart (36 floats per row: no bank conflicts);
+   * the others four rows at a time */
+  auto row_of = [&](int i) { return AK ? ty + 8 * i : (i < 4 ? ty * 4 + i : 28 + ty * 4 + i); };
+  auto col_of = [&](int j) { return BKm ? tx + 8 * j : (j < 4 ? tx * 4 + j : 28 + tx * 4 + j); };
+
+  const int slabs = (g.K + SK - 1) / SK, per = (slabs + n_split - 1) / n_split;
+  const int first = min(rank * per, slabs), n_slabs = min(first + per, slabs) - first;
+  const uint32_t smem = (uint32_t)__cvta_generic_to_shared(sm);
+  auto fetch = [&](int s) {
+    if (s < n_slabs) {
+      const uint32_t d = smem + (s % S_STAGES) * (2 * S_OPERAND * 4);
+      stage_operand<AK>(d, A, g.a_sm, g.a_sk, m0, g.M, (first + s) * SK, g.K, wide_a);
+      stage_operand<BKm>(d + S_OPERAND * 4, B, g.b_sn, g.b_sk, n0, g.N, (first + s) * SK, g.K, wide_b);
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  auto stash = [&](int buf) {
+  float acc[8][8];
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int e = tid + i * 256;
-      const int ka = a_kfast ? (e & 31) : (e >> 5), ma = a_kfast ? (e >> 5) : (e & 31);
-      const int kb = b_kfast ? (e & 31) : (e >> 5), nb = b_kfast ? (e >> 5) : (e & 31);
-      As[buf][ka][ma] = ra[i];
-      Bs[buf][kb][nb] = rb[i];
-    }
-  };
-  float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-  fetch(0);
-  stash(0);
-  __syncthreads();
-  const int nk = (g.K + SB - 1) / SB;
-  for (int kt = 0; kt < nk; kt++) {
-    const int cur = kt & 1;
-    if (kt + 1 < nk) fetch((kt + 1) * SB);
+  for (int i = 0; i < 8; i++)
 #pragma unroll
-    for (int k = 0; k < SB; k++) {
-      const float a0 = As[cur][k][ty * 2], a1 = As[cur][k][ty * 2 + 1];
-      const float b0 = Bs[cur][k][tx * 2], b1 = Bs[cur][k][tx * 2 + 1];
-      acc[0][0] = fmaf(a0, b0, acc[0][0]); acc[0][1] = fmaf(a0, b1, acc[0][1]);
-      acc[1][0] = fmaf(a1, b0, acc[1][0]); acc[1][1] = fmaf(a1, b1, acc[1][1]);
+    for (int j = 0; j < 8; j++) acc[i][j] = 0.0f;
+#pragma unroll
+  for (int s = 0; s < S_STAGES - 1; s++) fetch(s);
+  for (int s = 0; s < n_slabs; s++) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(S_STAGES - 2) : "memory");
+    __syncthreads();                                         /* slab s is there; slab s - 1 has been read by everyone */
+    fetch(s + S_STAGES - 1);
+    const float *as = sm + (s % S_STAGES) * (2 * S_OPERAND), *bs = as + S_OPERAND;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int k = (group + 4 * h) * 4;
+      float a[8][4], b[8][4];                                /* [row][k] */
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        if (AK) { const float4 v = *reinterpret_cast<const float4 *>(as + row_of(i) * (SK + 4) + k); a[i][0] = v.x; a[i][1] = v.y; a[i][2] = v.z; a[i][3] = v.w; }
+        else { const float4 v = *reinterpret_cast<const float4 *>(as + (k + (i & 3)) * (SB + 4) + (i >> 2) * 32 + ty * 4);
+               a[(i >> 2) * 4][i & 3] = v.x; a[(i >> 2) * 4 + 1][i & 3] = v.y; a[(i >> 2) * 4 + 2][i & 3] = v.z; a[(i >> 2) * 4 + 3][i & 3] = v.w; }
+        if (BKm) { const float4 v = *reinterpret_cast<const float4 *>(bs + col_of(i) * (SK + 4) + k); b[i][0] = v.x; b[i][1] = v.y; b[i][2] = v.z; b[i][3] = v.w; }
+        else { const float4 v = *reinterpret_cast<const float4 *>(bs + (k + (i & 3)) * (SB + 4) + (i >> 2) * 32 + tx * 4);
+               b[(i >> 2) * 4][i & 3] = v.x; b[(i >> 2) * 4 + 1][i & 3] = v.y; b[(i >> 2) * 4 + 2][i & 3] = v.z; b[(i >> 2) * 4 + 3][i & 3] = v.w; }
+      }
+#pragma unroll
+      for (int kk = 0; kk < 4; kk++)
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+#pragma unroll
+          for (int j = 0; j < 8; j++) acc[i][j] = fmaf(a[i][kk], b[j][kk], acc[i][j]);
     }
-    if (kt + 1 < nk) stash(cur ^ 1);
-    __syncthreads();
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; i++)
+#pragma unroll
+    for (int j = 0; j < 8; j++) sm[(group * SB + row_of(i)) * S_PITCH + col_of(j)] = acc[i][j];
+  __syncthreads();
+
   float *__restrict__ C = g.C + oc;
   const float *__restrict__ X = g.has_x ? g.X + ox : nullptr;
-#pragma unroll
-  for (int i = 0; i < 2; i++) {
-    const int m = m0 + ty * 2 + i;
-    if (m >= g.M) continue;
-#pragma unroll
-    for (int j = 0; j < 2; j++) {
-      const int n = n0 + tx * 2 + j;
-      if (n >= g.N) continue;
-      float t = __fmul_rn(acc[i][j], g.alpha);
-      if (X) t = t + X[(long long)m * g.x_sm + (long long)n * g.x_sn];
-      if (g.relu) t = (0.0f < t) ? t : 0.0f;
-      C[(long long)m * g.c_sm + (long long)n * g.c_sn] = t;
-    }
+  auto emit = [&](int r, int c, float sum) {
+    const int m = m0 + r, n = n0 + c;
+    if (m >= g.M || n >= g.N) return;
+    float t = __fmul_rn(sum, g.alpha);
+    if (X) t = t + X[(long long)m * g.x_sm + (long long)n * g.x_sn];
+    if (g.relu) t = (0.0f < t) ? t : 0.0f;
+    C[(long long)m * g.c_sm + (long long)n * g.c_sn] = t;
+  };
+  for (int e = threadIdx.x; e < SB * SB; e += 256) {
+    float *p = sm + (e / SB) * S_PITCH + e % SB;
+    const float sum = (p[0] + p[SB * S_PITCH]) + (p[2 * SB * S_PITCH] + p[3 * SB * S_PITCH]);
+    if (n_split == 1) emit(e / SB, e % SB, sum); else p[0] = sum;
   }
+  if (n_split == 1) return;
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  const int rows = SB / n_split;
+  for (int e = threadIdx.x; e < rows * SB; e += 256) {
+    const int r = rank * rows + e / SB, c = e % SB;
+    const uint32_t at = smem + (r * S_PITCH + c) * 4;
+    float v[8], sum = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      v[q] = 0.0f;
+      if (q < n_split) {
+        uint32_t peer;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(at), "r"(q));
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[q]) : "r"(peer) : "memory");
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 8; q++) if (q < n_split) sum = q ? sum + v[q] : v[q];
+    emit(r, c, sum);
+  }
+  /* no CTA leaves while another may still read its sums */
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <bool AK, bool BKm>
+static int small_launch(const SgemmArgs &g, dim3 grid, int n_split, bool wide_a, bool wide_b, cudaStream_t stream) {
+  static bool configured = false;
+  cudaError_t e = cudaSuccess;
+  if (!configured) { e = cudaFuncSetAttribute(pb200_sgemm_small<AK, BKm>, cudaFuncAttributeMaxDynamicSharedMemorySize, S_SMEM); configured = e == cudaSuccess; }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid.x * (unsigned)n_split, grid.y, grid.z); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = S_SMEM; cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)n_split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, pb200_sgemm_small<AK, BKm>, g, n_split, wide_a, wide_b);
+  if (e != cudaSuccess) { pb_set_error("sgemm launch: %s", cudaGetErrorString(e)); return -1; }
+  return 0;
 }
 
 static int sgemm_launch(const SgemmArgs &g, long long nbatch, cudaStream_t stream) {
-  /* fewer large tiles than SMs: the small-tile kernel spreads the work */
-  {
-    const long long big = (long long)((g.M + BM - 1) / BM) * ((g.N + BN - 1) / BN) * nbatch;
-    const long long small = (long long)((g.M + SB - 1) / SB) * ((g.N + SB - 1) / SB) * nbatch;
-    if (big < 74 && small <= 65535LL * 16 && nbatch <= 65535) {
-      dim3 grid((unsigned)((g.N + SB - 1) / SB), (unsigned)((g.M + SB - 1) / SB), (unsigned)nbatch);
-      if (grid.y <= 65535) {
-        pb200_sgemm_small<<<grid, 256, 0, stream>>>(g);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) { pb_set_error("sgemm launch: %s", cudaGetErrorString(e)); return -1; }
-        return 0;
-      }
-    }
-  }
-  /* operand layout: contiguous along k, or along the row/column axis */
-  const bool a_k = (g.a_sk == 1) || g.K == 1, b_k = (g.b_sk == 1 && g.b_sn != 1);
-  const bool a_ok = a_k ? true : (g.a_sm == 1), b_ok = b_k ? true : (g.b_sn == 1);
   auto aligned = [](const void *p, long long ld, const long long *sb, int nb) {
     if (reinterpret_cast<uintptr_t>(p) & 15) return false;
     if (ld & 3) return false;
     for (int i = 0; i < nb; i++) if (sb[i] & 3) return false;
     return true;
   };
+  /* fewer large tiles than half the SMs: small tiles, their k axis split between as many CTAs as keep the SMs busy.
+   * Estimated in clocks: a slab of a tile, the start and the two reductions of a CTA. */
+  {
+    const long long big = (long long)((g.M + BM - 1) / BM) * ((g.N + BN - 1) / BN) * nbatch;
+    const long long tn = (g.N + SB - 1) / SB, tm = (g.M + SB - 1) / SB, tiles = tm * tn * nbatch;
+    if (big < 74 && tm <= 65535 && nbatch <= 65535) {
+      const long long slabs = ((long long)g.K + SK - 1) / SK;
+      int n_split = 1;
+      long long best = -1;
+      for (int s = 1; s <= 8; s *= 2) {
+        const long long cost = ((tiles * s + 147) / 148) * ((slabs + s - 1) / s * 1200 + (s > 1 ? 4500 : 3500));
+        if (best < 0 || cost < best) { best = cost; n_split = s; }
+      }
+      const bool ak = g.a_sk == 1, bk = g.b_sk == 1 && g.b_sn != 1;
+      const bool wa = (ak || g.a_sm == 1) && aligned(g.A, ak ? g.a_sm : g.a_sk, g.a_sb, g.nb);
+      const bool wb = (bk || g.b_sn == 1) && aligned(g.B, bk ? g.b_sn : g.b_sk, g.b_sb, g.nb);
+      const dim3 grid((unsigned)tn, (unsigned)tm, (unsigned)nbatch);
+      if (ak) return bk ? small_launch<true, true>(g, grid, n_split, wa, wb, stream) : small_launch<true, false>(g, grid, n_split, wa, wb, stream);
+      return bk ? small_launch<false, true>(g, grid, n_split, wa, wb, stream) : small_launch<false, false>(g, grid, n_split, wa, wb, stream);
+    }
+  }
+  /* operand layout: contiguous along k, or along the row/column axis */
+  const bool a_k = (g.a_sk == 1) || g.K == 1, b_k = (g.b_sk == 1 && g.b_sn != 1);
+  const bool a_ok = a_k ? true : (g.a_sm == 1), b_ok = b_k ? true : (g.b_sn == 1);
   const bool va = a_ok && aligned(g.A, a_k ? g.a_sm : g.a_sk, g.a_sb, g.nb);
   const bool vb = b_ok && aligned(g.B, b_k ? g.b_sn : g.b_sk, g.b_sb, g.nb);
   SgemmFn fn;

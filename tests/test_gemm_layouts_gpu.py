@@ -106,3 +106,23 @@ def test_rows_of_float32_off_the_16_byte_grid(kernels, m, n, k, relu):  # noqa: 
     got, want = kernels.get(c, (m, n)), a @ b.T
     for r in range(0, m, 500):
         assert_close(got[r:r + 500], np.maximum(want[r:r + 500], 0) if relu else want[r:r + 500], 1e-4, f'{m} {n} {k} from row {r}')
+
+
+SMALL = [(1, 1, 1), (256, 10, 512), (64, 64, 32), (65, 63, 33), (3, 200, 5000), (100, 1, 77), (1, 100, 64), (256, 512, 784), (500, 900, 100)]
+
+
+@pytest.mark.parametrize('pad', [0, 4, 3])
+@pytest.mark.parametrize('a_kfast,b_kfast', [(True, False), (True, True), (False, False), (False, True)])
+@pytest.mark.parametrize('m,n,k', SMALL, ids=str)
+def test_small_f32(kernels, m, n, k, a_kfast, b_kfast, pad):  # noqa: F811
+    """One to eight CTAs per tile, slabs of k that are missing, partial or past the end, every operand order and
+    alignment; the sums are float32 ones in another order than float64's, far inside 1e-5 at these K."""
+    rng = np.random.default_rng([m, n, k, pad])
+    a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
+    bias = rng.standard_normal(n).astype(np.float32)
+    ma, (a_sm, a_sk) = stored(a, a_kfast, pad, rng, lambda x: x)
+    mb, (b_sn, b_sk) = stored(b, b_kfast, pad, rng, lambda x: x)
+    c = kernels.put(np.zeros((m, n), np.float32))
+    assert kernels.c.poly_b200_gemm(m, n, k, kernels.put(ma), a_sm, a_sk, kernels.put(mb), b_sk, b_sn, c, n, kernels.put(bias), 1, 0) == 0, kernels.error()
+    want = np.maximum(a.astype(np.float64) @ b.T.astype(np.float64) + bias, 0)
+    assert_close(kernels.get(c, (m, n)), want, 1e-5, f'f32 {m} {n} {k}')
