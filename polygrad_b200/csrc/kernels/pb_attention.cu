@@ -65,6 +65,20 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
+/* x = fma(s, scale, mask) for 32 keys of a thread's row; the mask row lies in shared memory as eight 16-byte chunks,
+ * chunk i at i ^ swz */
+__device__ __forceinline__ void add_mask_row(uint32_t (&r)[32], uint32_t row, int swz, float scale) {
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    float a, b, c, d;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(a), "=f"(b), "=f"(c), "=f"(d) : "r"(row + ((i ^ swz) << 4)) : "memory");
+    r[4 * i] = __float_as_uint(fmaf(__uint_as_float(r[4 * i]), scale, a));
+    r[4 * i + 1] = __float_as_uint(fmaf(__uint_as_float(r[4 * i + 1]), scale, b));
+    r[4 * i + 2] = __float_as_uint(fmaf(__uint_as_float(r[4 * i + 2]), scale, c));
+    r[4 * i + 3] = __float_as_uint(fmaf(__uint_as_float(r[4 * i + 3]), scale, d));
+  }
+}
+
 struct AttnArgs {
   float *O; const float *mask;
   long long mask_sq, mask_sk;     /* mask[q*mask_sq + k*mask_sk] */
@@ -553,13 +567,54 @@ pb200_flash_attn2(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       const uint32_t ph = it & 1u;
       const float tile_c = s_tc[j];
       const bool tile_is_const = (tile_c == tile_c), tile_is_step = s_kind[j] == 2.0f;
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_s, ph, &abort_flag, 17))) { ok = false; break; }
-      tc_fence_after_sync();
-      /* this thread's 64 scores, once */
+      const bool staged = !tile_is_const && !tile_is_step && g.mask_vec;
       uint32_t r0[32], r1[32];
-      tc_ld32(s_cols, r0);
-      tc_ld32(s_cols + 32, r1);
-      tc_wait_ld();
+      if (staged) {
+        /* A mask tile of its own values.  The warp fetches its 32 rows x 64 keys in whole 128-byte lines and turns
+         * them through its 4 KB of the P tile (idle between the previous block's product and this block's
+         * probabilities): the first 32 keys copied there asynchronously, the others held in registers meanwhile.
+         * Read by each thread along its own row, 32 rows per instruction, 1 x 25 x 2048 x 64 with a position bias
+         * took 249 us, most of it in the L1's line lookups; 188 like this (pb200_attn_prepare included). */
+        if (it > 0 && !__all_sync(0xffffffffu, mbar_wait(bar_o, (it - 1) & 1u, &abort_flag, 18))) { ok = false; break; }
+        const uint32_t stg = s_p + half * 16384 + quarter * 4096;
+        const int sub = lane & 7, rr = lane >> 3;
+        const float *mw = g.mask + ((long long)qb * AT_BQ + quarter * 32 + rr) * g.mask_sq + (long long)j * AT_BK + half * 64 + sub * 4;
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const int r = rr + 4 * i;
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(stg + r * 128 + ((sub ^ (r & 7)) << 4)), "l"(mw + (long long)(4 * i) * g.mask_sq) : "memory");
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const float4 v = __ldg(reinterpret_cast<const float4 *>(mw + (long long)(4 * i) * g.mask_sq + 32));
+          r1[4 * i] = __float_as_uint(v.x); r1[4 * i + 1] = __float_as_uint(v.y); r1[4 * i + 2] = __float_as_uint(v.z); r1[4 * i + 3] = __float_as_uint(v.w);
+        }
+        if (!__all_sync(0xffffffffu, mbar_wait(bar_s, ph, &abort_flag, 17))) { ok = false; break; }
+        tc_fence_after_sync();
+        tc_ld32(s_cols, r0);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+        tc_wait_ld();
+        add_mask_row(r0, stg + lane * 128, lane & 7, g.scale);
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const int r = rr + 4 * i;
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stg + r * 128 + ((sub ^ (r & 7)) << 4)), "r"(r1[4 * i]), "r"(r1[4 * i + 1]), "r"(r1[4 * i + 2]), "r"(r1[4 * i + 3]) : "memory");
+        }
+        tc_ld32(s_cols + 32, r1);
+        __syncwarp();
+        tc_wait_ld();
+        add_mask_row(r1, stg + lane * 128, lane & 7, g.scale);
+      } else {
+        if (!__all_sync(0xffffffffu, mbar_wait(bar_s, ph, &abort_flag, 17))) { ok = false; break; }
+        tc_fence_after_sync();
+        /* this thread's 64 scores, once */
+        tc_ld32(s_cols, r0);
+        tc_ld32(s_cols + 32, r1);
+        tc_wait_ld();
+      }
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_f);
@@ -570,7 +625,10 @@ pb200_flash_attn2(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       const bool plain = tile_is_const && g.scale >= 0.0f, step = tile_is_step && g.scale >= 0.0f;
       const float lo = s_lo[j], hi = s_hi[j];
       const int thr = (int)s_d[j] + row - half * 64;        /* key k of the thread's 64 has the value lo where k > thr, else hi */
-      if (plain) {
+      if (staged) {
+#pragma unroll
+        for (int i = 0; i < 32; i++) m_part = fmaxf(m_part, fmaxf(__uint_as_float(r0[i]), __uint_as_float(r1[i])));
+      } else if (plain) {
 #pragma unroll
         for (int i = 0; i < 32; i++) m_part = fmaxf(m_part, fmaxf(__uint_as_float(r0[i]), __uint_as_float(r1[i])));
         m_part = fmaf(m_part, g.scale, tile_c);
@@ -597,15 +655,6 @@ pb200_flash_attn2(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             /* (negative scale) the entries of a step tile from the indices: no loads */
 #pragma unroll
             for (int i = 0; i < 32; i++) r[i] = __float_as_uint(fmaf(__uint_as_float(r[i]), g.scale, (c * 32 + i > thr) ? lo : hi));
-          } else if (g.mask_vec) {
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-              const float4 mv = reinterpret_cast<const float4 *>(mj + c * 32)[i];
-              r[4 * i] = __float_as_uint(fmaf(__uint_as_float(r[4 * i]), g.scale, mv.x));
-              r[4 * i + 1] = __float_as_uint(fmaf(__uint_as_float(r[4 * i + 1]), g.scale, mv.y));
-              r[4 * i + 2] = __float_as_uint(fmaf(__uint_as_float(r[4 * i + 2]), g.scale, mv.z));
-              r[4 * i + 3] = __float_as_uint(fmaf(__uint_as_float(r[4 * i + 3]), g.scale, mv.w));
-            }
           } else {
 #pragma unroll
             for (int i = 0; i < 32; i++)
@@ -748,8 +797,7 @@ pb200_flash_attn2(const __grid_constant__ CUtensorMap map_q, const __grid_consta
  *       (the diagonal tiles of a causal mask: -1e9 above the diagonal, 0 on and below it), so
  *       that the kernel forms the entries from the indices instead of loading 64 KB; else 0.
  * Every claim is checked bit for bit against all 16384 entries: exact for every mask. */
-__global__ void __launch_bounds__(256) pb200_mask_tiles(const float *mask, long long sq, long long sk, int nk, float *out) {
-  const int qi = blockIdx.y, ki = blockIdx.x;
+__device__ __forceinline__ void mask_tile(const float *mask, long long sq, long long sk, int nk, float *out, int qi, int ki) {
   const float *t = mask + (long long)qi * AT_BQ * sq + (long long)ki * AT_BK * sk;
   const float first = t[0];
   /* step hypothesis from the corners and from row 0: lo = top right, hi = bottom left, and row 0 holds hi in
@@ -813,6 +861,76 @@ __global__ void __launch_bounds__(256) pb200_mask_tiles(const float *mask, long 
     /* a step tile has two different finite-or-infinite values (NaNs are left to the general path) */
     rec[2] = (!is_const && step && lo == lo && hi == hi && lo_b != hi_b) ? 2.0f : 0.0f;
     rec[3] = (float)d; rec[4] = lo; rec[5] = hi; rec[6] = 0.0f; rec[7] = 0.0f;
+  }
+}
+
+__global__ void __launch_bounds__(256) pb200_mask_tiles(const float *mask, long long sq, long long sk, int nk, float *out) {
+  mask_tile(mask, sq, sk, nk, out, blockIdx.y, blockIdx.x);
+}
+
+/* Everything the attention kernel needs of float32 operands, in one launch: the first nq * nk blocks classify the
+ * mask's tiles; each of the others rounds 128 rows of one head of q, k and v to bfloat16 (same [B][T][H][64] layout)
+ * and bounds the norms of the rounded q and k rows while they are in registers.  Bound by memory (4 bytes read, 2
+ * written per element).  (Three conversions, the bounds and the classification were five
+ * launches: 8 x 12 x 1024 x 64 with a causal mask took 115.5 us in all, 89 like this.) */
+struct PrepareArgs {
+  const float *src[3]; __nv_bfloat16 *dst[3];
+  int H, T, nblk; long long D;
+  float *qn, *kn;                 /* null: no bounds wanted */
+  const float *mask; int nk; float *tiles; int n_mask;
+};
+__global__ void __launch_bounds__(256) pb200_attn_prepare(const PrepareArgs a) {
+  if ((int)blockIdx.x < a.n_mask) { mask_tile(a.mask, a.T, 1, a.nk, a.tiles, blockIdx.x / a.nk, blockIdx.x % a.nk); return; }
+  const int id = blockIdx.x - a.n_mask, blk = id % a.nblk, bh = id / a.nblk;
+  /* 8 threads per row of 64, 32 rows per pass */
+  const int sub = threadIdx.x & 7, grp = threadIdx.x >> 3;
+  const long long at = ((long long)(bh / a.H) * a.T + blk * 128 + grp) * a.D + (bh % a.H) * AT_HD + sub * 8;
+  __shared__ float s_max[2][8];
+#pragma unroll
+  for (int t = 0; t < 3; t++) {
+    const float *src = a.src[t] + at;
+    __nv_bfloat16 *dst = a.dst[t] + at;
+    float4 v[8];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      v[2 * i] = __ldg(reinterpret_cast<const float4 *>(src + i * 32 * a.D));
+      v[2 * i + 1] = __ldg(reinterpret_cast<const float4 *>(src + i * 32 * a.D + 4));
+    }
+    float big = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const __nv_bfloat162 p[4] = {__floats2bfloat162_rn(v[2 * i].x, v[2 * i].y), __floats2bfloat162_rn(v[2 * i].z, v[2 * i].w),
+                                   __floats2bfloat162_rn(v[2 * i + 1].x, v[2 * i + 1].y), __floats2bfloat162_rn(v[2 * i + 1].z, v[2 * i + 1].w)};
+      uint4 w;
+      w.x = *reinterpret_cast<const uint32_t *>(&p[0]); w.y = *reinterpret_cast<const uint32_t *>(&p[1]);
+      w.z = *reinterpret_cast<const uint32_t *>(&p[2]); w.w = *reinterpret_cast<const uint32_t *>(&p[3]);
+      *reinterpret_cast<uint4 *>(dst + i * 32 * a.D) = w;
+      if (t < 2 && a.qn) {
+        float sq = 0.0f;
+#pragma unroll
+        for (int c = 0; c < 4; c++) { const float2 x = __bfloat1622float2(p[c]); sq = fmaf(x.x, x.x, fmaf(x.y, x.y, sq)); }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        big = (big != big || sq != sq) ? __int_as_float(0x7fc00000) : fmaxf(big, sq);
+      }
+    }
+    if (t < 2 && a.qn) {
+      /* NaN rows give NaN norms, and a NaN bound never permits a skip */
+#pragma unroll
+      for (int o = 8; o < 32; o <<= 1) {
+        const float x = __shfl_xor_sync(0xffffffffu, big, o);
+        big = (big != big || x != x) ? __int_as_float(0x7fc00000) : fmaxf(big, x);
+      }
+      if ((threadIdx.x & 31) == 0) s_max[t][threadIdx.x >> 5] = big;
+    }
+  }
+  if (!a.qn) return;
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    float x = s_max[threadIdx.x][0];
+    for (int i = 1; i < 8; i++) { const float y = s_max[threadIdx.x][i]; x = (x != x || y != y) ? __int_as_float(0x7fc00000) : fmaxf(x, y); }
+    /* rounded up: the sums above and the tensor cores' own accumulation round */
+    (threadIdx.x ? a.kn : a.qn)[(long long)bh * a.nblk + blk] = sqrtf(x) * 1.001f;
   }
 }
 
@@ -924,10 +1042,13 @@ bool pb_attention_supported(long long T, long long hd) { return hd == AT_HD && T
 
 /* q, k, v: bf16 through strides; mask fp32 [T x T] through strides; out fp32 or bf16 (out_bf16)
  * at element offsets Σ batch_i*o_sb[i] + row*o_sm + d. */
+/* POLY_B200_ATTN_SKIP=0: no key block is left out */
+static bool attn_skips() { const char *e = getenv("POLY_B200_ATTN_SKIP"); return !(e && e[0] == '0'); }
+
 int pb_attention_launch(const PbAttnOperand &q, const PbAttnOperand &k, const PbAttnOperand &v,
                         const float *mask, long long mask_sq, long long mask_sk,
                         float scale, void *out, bool out_bf16, int nb, const int *bext, const long long *o_sb, long long o_sm,
-                        long long BH, long long T, cudaStream_t stream, float *tiles_buf, int tiles_mode) {
+                        long long BH, long long T, cudaStream_t stream, float *tiles_buf, int tiles_mode, const float *norms_ready) {
   if (!pb_attention_supported(T, AT_HD)) { pb_set_error("attention: unsupported sequence length %lld", T); return -1; }
   if (nb > 3) { pb_set_error("attention: more than three batch axes"); return -1; }
   const int oal = out_bf16 ? 8 : 4;
@@ -961,9 +1082,9 @@ int pb_attention_launch(const PbAttnOperand &q, const PbAttnOperand &k, const Pb
   if (!tiles) { pb_set_error("attention: out of scratch memory"); return -1; }
   /* bounds on |q.k| per block, for leaving out key blocks that cannot contribute (POLY_B200_ATTN_SKIP=0: never) */
   float *norms = nullptr;
-  {
-    const char *e = getenv("POLY_B200_ATTN_SKIP");
-    if (!(e && e[0] == '0')) {
+  if (norms_ready) { g.qn = norms_ready; g.kn = norms_ready + BH * nq; }
+  else {
+    if (attn_skips()) {
       norms = (float *)pb_scratch_alloc((size_t)2 * BH * nq * sizeof(float));
       if (!norms) { if (!tiles_mode) pb_scratch_free(tiles); pb_set_error("attention: out of scratch memory"); return -1; }
       BoundsArgs ba{};
@@ -988,6 +1109,8 @@ int pb_attention_launch(const PbAttnOperand &q, const PbAttnOperand &k, const Pb
   return 0;
 }
 
+static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
 /* Direct entry: q, k, v float32 [B][T][H][64] (the layout GPT-2's projections
  * produce), mask float32 [T][T], out float32 [B][H][T][64]. */
 extern "C" int poly_b200_attention(const float *q, const float *k, const float *v, const float *mask, float scale,
@@ -1001,9 +1124,27 @@ extern "C" int poly_b200_attention(const float *q, const float *k, const float *
   if (pb_note_read(q) != 0 || pb_note_read(k) != 0 || pb_note_read(v) != 0 || pb_note_read(mask) != 0 ||
       pb_note_write(out, (size_t)BH * T * AT_HD * 4) != 0) return -1;
   void *qb = pb_scratch_alloc(bytes), *kb = pb_scratch_alloc(bytes), *vb = pb_scratch_alloc(bytes);
+  const long long nq = T / AT_BQ, n_blocks = BH * nq + nq * nq;
+  /* mask records, then the norms of q's and of k's blocks */
+  float *records = aligned16(q) && aligned16(k) && aligned16(v) && n_blocks <= 2147483647LL
+                       ? (float *)pb_scratch_alloc((size_t)(AT_REC * nq * nq + 2 * BH * nq) * sizeof(float)) : nullptr;
   int rc = -1;
-  if (qb && kb && vb) {
-    /* fp32 [b][t][h][d] -> bf16 in the same layout */
+  if (qb && kb && vb && records) {
+    PrepareArgs a{};
+    a.src[0] = q; a.src[1] = k; a.src[2] = v;
+    a.dst[0] = (__nv_bfloat16 *)qb; a.dst[1] = (__nv_bfloat16 *)kb; a.dst[2] = (__nv_bfloat16 *)vb;
+    a.H = H; a.T = T; a.nblk = (int)nq; a.D = D;
+    float *norms = records + AT_REC * nq * nq;
+    if (attn_skips()) { a.qn = norms; a.kn = norms + BH * nq; }
+    a.mask = mask; a.nk = (int)nq; a.tiles = records; a.n_mask = (int)(nq * nq);
+    pb200_attn_prepare<<<(unsigned)n_blocks, 256, 0, stream>>>(a);
+    const int bext[2] = {H, B};
+    const long long o_sb[2] = {(long long)T * AT_HD, (long long)H * T * AT_HD};
+    PbAttnOperand oq{qb, D, {AT_HD, (long long)T * D, 0}}, ok{kb, D, {AT_HD, (long long)T * D, 0}}, ov{vb, D, {AT_HD, (long long)T * D, 0}};
+    rc = pb_attention_launch(oq, ok, ov, mask, T, 1, scale, out, false, 2, bext, o_sb, AT_HD, BH, T, stream, records, 2, a.qn);
+    if (rc == 0) pb_count_launch(true, 2);
+  } else if (qb && kb && vb) {
+    /* operands off the 16-byte grid: fp32 [b][t][h][d] -> bf16 in the same layout */
     const long long ext[2] = {D, (long long)B * T}, str[2] = {1, D};
     rc = pb_pack_launch(q, qb, 2, ext, str, PB_F32, PB_BF16, D, D, stream);
     if (rc == 0) rc = pb_pack_launch(k, kb, 2, ext, str, PB_F32, PB_BF16, D, D, stream);
@@ -1014,7 +1155,7 @@ extern "C" int poly_b200_attention(const float *q, const float *k, const float *
     if (rc == 0) rc = pb_attention_launch(oq, ok, ov, mask, T, 1, scale, out, false, 2, bext, o_sb, AT_HD, BH, T, stream);
     if (rc == 0) pb_count_launch(true, 4);
   } else pb_set_error("poly_b200_attention: out of scratch memory");
-  pb_scratch_free(qb); pb_scratch_free(kb); pb_scratch_free(vb);
+  pb_scratch_free(qb); pb_scratch_free(kb); pb_scratch_free(vb); pb_scratch_free(records);
   return rc;
 }
 

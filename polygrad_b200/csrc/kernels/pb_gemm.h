@@ -66,9 +66,11 @@ struct PbAttnOperand { const void *ptr; long long row_stride; long long bstride[
 int pb_attention_launch(const PbAttnOperand &q, const PbAttnOperand &k, const PbAttnOperand &v,
                         const float *mask, long long mask_sq, long long mask_sk,
                         float scale, void *out, bool out_bf16, int nb, const int *bext, const long long *o_sb, long long o_sm,
-                        long long BH, long long T, cudaStream_t stream, float *tiles = nullptr, int tiles_mode = 0);
+                        long long BH, long long T, cudaStream_t stream, float *tiles = nullptr, int tiles_mode = 0,
+                        const float *norms_ready = nullptr);
 /* tiles_mode 1: the mask classification (a record of eight floats per 128 x 128 tile of the mask) is computed into `tiles`,
- * 2: it is read from there; 0: the launch uses scratch of its own. */
+ * 2: it is read from there; 0: the launch uses scratch of its own.  norms_ready: the row-norm bounds of q's blocks and
+ * then of k's, where they have been computed already. */
 
 /* Can the tensor-core kernel run this problem whatever the buffer addresses are
  * (16-byte aligned bases assumed), reading A in place when a_bf16 and writing
