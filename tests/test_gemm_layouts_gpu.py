@@ -126,3 +126,18 @@ def test_small_f32(kernels, m, n, k, a_kfast, b_kfast, pad):  # noqa: F811
     assert kernels.c.poly_b200_gemm(m, n, k, kernels.put(ma), a_sm, a_sk, kernels.put(mb), b_sk, b_sn, c, n, kernels.put(bias), 1, 0) == 0, kernels.error()
     want = np.maximum(a.astype(np.float64) @ b.T.astype(np.float64) + bias, 0)
     assert_close(kernels.get(c, (m, n)), want, 1e-5, f'f32 {m} {n} {k}')
+
+
+@pytest.mark.parametrize('pad', [0, 4, 3])
+@pytest.mark.parametrize('a_kfast,b_kfast', [(True, False), (True, True), (False, False), (False, True)])
+@pytest.mark.parametrize('m,n,k', SIZES, ids=str)
+def test_f32_operands_rounded_to_bf16(kernels, m, n, k, a_kfast, b_kfast, pad):  # noqa: F811
+    kernels.c.poly_b200_set_gemm_policy(1)
+    rng = np.random.default_rng([m, n, k, pad])
+    a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
+    ma, (a_sm, a_sk) = stored(a, a_kfast, pad, rng, lambda x: x)
+    mb, (b_sn, b_sk) = stored(b, b_kfast, pad, rng, lambda x: x)
+    c = kernels.put(np.zeros((m, n), np.float32))
+    assert kernels.c.poly_b200_gemm(m, n, k, kernels.put(ma), a_sm, a_sk, kernels.put(mb), b_sk, b_sn, c, n, None, 0, 0) == 0, kernels.error()
+    want = bf16(a).astype(np.float64) @ bf16(b).T.astype(np.float64)
+    assert_close(kernels.get(c, (m, n)), want, 1e-4, f'policy {m} {n} {k}')
