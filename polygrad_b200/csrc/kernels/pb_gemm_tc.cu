@@ -127,14 +127,14 @@ __device__ __forceinline__ void tile_coords(const TcArgs &g, int t, int *mt, int
 
 /* CTAS = 2: two CTAs on neighbouring SMs (a cluster of 2) work on one 256 x BN tile with
  * cta_group::2 MMAs; each holds its 128 rows of A and half of the tile's B rows. */
-template <int BN, int CTAS, bool TF32 = false>
+template <int BN, int CTAS, bool TF32 = false, bool RING = false>
 struct TcSmem {
   static constexpr int PARTS = TF32 ? 2 : 1;                 /* a float32 operand comes as two tf32 tiles, hi and lo */
   static constexpr int STAGE_A = TC_BM * TC_BK * 2 * PARTS;
   static constexpr int STAGE_B = (BN / CTAS) * TC_BK * 2 * PARTS;
   static constexpr int STAGE = STAGE_A + STAGE_B;
-  static constexpr int STAGES = TF32 ? 196608 / STAGE : CTAS == 2 ? (BN >= 192 ? 6 : 8) : ((BN == 256) ? 4 : (BN == 192 ? 4 : (BN == 128 ? 6 : 8)));
-  static constexpr int EPI = 8 * 32 * 32 * 4;
+  static constexpr int STAGES = RING ? 163840 / STAGE : TF32 ? 196608 / STAGE : CTAS == 2 ? (BN >= 192 ? 6 : 8) : ((BN == 256) ? 4 : (BN == 192 ? 4 : (BN == 128 ? 6 : 8)));
+  static constexpr int EPI = 8 * 32 * 32 * 4 * (RING ? 2 : 1);      /* staging tiles of the epilogue warps */
   static constexpr int BYTES = STAGES * STAGE + EPI + 256 + 1024; /* + barriers + alignment slack */
 };
 
@@ -142,10 +142,10 @@ struct TcSmem {
 
 /* MN: an operand may have contiguous rows (a_mn, b_mn); without it the kernel is compiled for k-contiguous ones alone,
  * which keeps the issuing threads of short contractions free of the choice (197 x 2304 x 768: 1 us). */
-template <int BN, int CTAS, bool PROMOTE = false, bool TF32 = false, bool MN = false>
+template <int BN, int CTAS, bool PROMOTE = false, bool TF32 = false, bool MN = false, bool RING = false>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 pb200_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const TcArgs g) {
-  using S = TcSmem<BN, CTAS, TF32>;
+  using S = TcSmem<BN, CTAS, TF32, RING>;
   static_assert(S::BYTES <= 227 * 1024 - 64, "shared memory");
   /* CTA pair: rank within the pair, the pair's index and count (tiles are handed out per pair) */
   const uint32_t rank = CTAS == 2 ? cluster_ctarank() : 0u;
@@ -318,7 +318,7 @@ pb200_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
     /* ── epilogue: 8 warps; warp w reads tensor-memory lanes 32*(w%4) .. +31 (the
      * hardware ties a warp to that quarter) and one half of the tile's columns ── */
     const int q = warp & 3, half = (warp - 2) >> 2;
-    float *stg = epi + (warp - 2) * 32 * 32;
+    float *stg = epi + (warp - 2) * 32 * 32 * (RING ? 2 : 1);
     /* addresses into this warp's 4 KB staging tile, fixed for the whole kernel.  float32 tile: 32 rows x 128 B,
      * thread `lane` writes row `lane` (16-byte chunk c at c ^ (lane & 7)) and reads, in pass i8, row i8*4 + lane/8,
      * chunk lane%8.  bfloat16 tile: 32 rows x 64 B, chunk c of row r at c ^ ((r >> 1) & 3); pass i4 reads row
@@ -411,6 +411,52 @@ pb200_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
         if constexpr (PROMOTE) return acc[ci][j] * g.alpha; else return __uint_as_float(r[ci & 1][j]);
       };
       if constexpr (!PROMOTE) { if (colh < g.N) tc_ld32(tbase, r[0]); }
+      if constexpr (RING) {
+        /* Rows that start anywhere, float32, no addend.  A 128-byte store at a row's own offset touches two lines and
+         * leaves sectors half written; so two chunks are staged at a time (a row is 64 words, 16-byte chunk c of
+         * row r at c + r mod 16: no bank conflicts either way), and what goes out is, row by row, the whole line
+         * that the newest chunk completes.  8192 x 50257 x 768: 900 -> 845 us. */
+        const int lim = max(0, min(g.N - colh, BN / 2));       /* columns of this warp's part */
+        const uint32_t s0 = (uint32_t)((reinterpret_cast<uintptr_t>(C + (long long)row0 * g.c_sm + colh) >> 2) & 31), cs = (uint32_t)g.c_sm & 31;
+        const uint32_t wr = stg_s + lane * 256;
+#pragma unroll
+        for (int ci = 0; ci <= NCH; ci++) {
+          if (lim > 0 && ci * 32 - 31 < lim) {
+            __syncwarp();                                      /* the slot's previous chunk has been read */
+            if (ci < NCH && ci * 32 < lim) {
+              tc_wait_ld();
+              if (ci + 1 < NCH && ci * 32 + 32 < lim) tc_ld32(tbase + (ci + 1) * 32, r[(ci + 1) & 1]);
+#pragma unroll
+              for (int c = 0; c < 8; c++)
+                sts_v4(wr + ((((ci & 1) * 8 + c + lane) & 15) << 4), r[ci & 1][c * 4], r[ci & 1][c * 4 + 1], r[ci & 1][c * 4 + 2], r[ci & 1][c * 4 + 3]);
+            }
+            __syncwarp();
+            float *row = C + (long long)row0 * g.c_sm + colh;
+            auto emit = [&](auto relu, auto cs_store) {
+#pragma unroll
+              for (int r16 = 0; r16 < 2; r16++) {
+                uint32_t v[16]; int p[16];
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                  const int rr = r16 * 16 + i;
+                  p[i] = ci * 32 + lane - (int)((s0 + rr * cs) & 31);                       /* column within the warp's part */
+                  v[i] = lds_b32(stg_s + rr * 256 + (((p[i] + 4 * rr) & 63) << 2));
+                }
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                  float a = __uint_as_float(v[i]) + 0.0f;
+                  if (decltype(relu)::value) a = (0.f < a) ? a : 0.f;
+                  if ((uint32_t)p[i] < (uint32_t)lim && r16 * 16 + i < rows) { if (decltype(cs_store)::value) stg_b32_cs(row + p[i], __float_as_uint(a)); else stg_b32(row + p[i], __float_as_uint(a)); }
+                  row += g.c_sm;
+                }
+              }
+            };
+            if (g.relu) { if (g.stream_out) emit(std::true_type(), std::true_type()); else emit(std::true_type(), std::false_type()); }
+            else { if (g.stream_out) emit(std::false_type(), std::true_type()); else emit(std::false_type(), std::false_type()); }
+          }
+        }
+        __syncwarp();
+      } else
 #pragma unroll
       for (int ci = 0; ci < NCH; ci++) {
         const int col0 = colh + ci * 32;
@@ -659,12 +705,12 @@ static int make_map(CUtensorMap *map, const void *ptr, long long K, long long ro
 }
 
 /* One-time set-up of a kernel variant (the runtime drives one device per process). */
-template <int BN, int CTAS, bool PROMOTE = false, bool TF32 = false, bool MN = false>
+template <int BN, int CTAS, bool PROMOTE = false, bool TF32 = false, bool MN = false, bool RING = false>
 static int tc_configure() {
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(pb200_gemm_tc<BN, CTAS, PROMOTE, TF32, MN>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcSmem<BN, CTAS, TF32>::BYTES);
-    if (e != cudaSuccess) { pb_set_error("gemm: cannot reserve %d bytes of shared memory: %s", TcSmem<BN, CTAS, TF32>::BYTES, cudaGetErrorString(e)); return -1; }
+    cudaError_t e = cudaFuncSetAttribute(pb200_gemm_tc<BN, CTAS, PROMOTE, TF32, MN, RING>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcSmem<BN, CTAS, TF32, RING>::BYTES);
+    if (e != cudaSuccess) { pb_set_error("gemm: cannot reserve %d bytes of shared memory: %s", TcSmem<BN, CTAS, TF32, RING>::BYTES, cudaGetErrorString(e)); return -1; }
     configured = true;
   }
   return 0;
@@ -676,9 +722,9 @@ static int sm_count() {
   return sms;
 }
 
-template <int BN, int CTAS, bool PROMOTE = false, bool TF32 = false, bool MN = false>
+template <int BN, int CTAS, bool PROMOTE = false, bool TF32 = false, bool MN = false, bool RING = false>
 static int tc_launch(const CUtensorMap &ma, const CUtensorMap &mb, TcArgs &g, long long nbatch, cudaStream_t stream) {
-  if (tc_configure<BN, CTAS, PROMOTE, TF32, MN>() != 0) return -1;
+  if (tc_configure<BN, CTAS, PROMOTE, TF32, MN, RING>() != 0) return -1;
   g.tiles_m = (g.M + TC_BM * CTAS - 1) / (TC_BM * CTAS);
   g.tiles_n = (g.N + BN - 1) / BN;
   long long tiles = (long long)g.tiles_m * g.tiles_n * nbatch;
@@ -693,23 +739,34 @@ static int tc_launch(const CUtensorMap &ma, const CUtensorMap &mb, TcArgs &g, lo
   const int grid = (int)(tiles < units ? tiles : units) * CTAS;
   cudaError_t e;
   if (CTAS == 1) {
-    pb200_gemm_tc<BN, CTAS, PROMOTE, TF32, MN><<<grid, TC_THREADS, TcSmem<BN, CTAS, TF32>::BYTES, stream>>>(ma, mb, g);
+    pb200_gemm_tc<BN, CTAS, PROMOTE, TF32, MN, RING><<<grid, TC_THREADS, TcSmem<BN, CTAS, TF32, RING>::BYTES, stream>>>(ma, mb, g);
     e = cudaGetLastError();
   } else {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid); cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = TcSmem<BN, CTAS, TF32>::BYTES; cfg.stream = stream;
+    cfg.gridDim = dim3((unsigned)grid); cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = TcSmem<BN, CTAS, TF32, RING>::BYTES; cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = CTAS; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, pb200_gemm_tc<BN, CTAS, PROMOTE, TF32, MN>, ma, mb, g);
+    e = cudaLaunchKernelEx(&cfg, pb200_gemm_tc<BN, CTAS, PROMOTE, TF32, MN, RING>, ma, mb, g);
   }
   if (e != cudaSuccess) { pb_set_error("tensor-core gemm launch: %s", cudaGetErrorString(e)); return -1; }
   return 0;
 }
 
+/* Result rows of any alignment that are written line by line (RING), by CTA pairs: whole lines need a second staging tile
+ * per warp, which a pair's smaller stages leave room for.  From 74 pair tiles on (8192 x 50257 x 768: 845 us, pairs that store 32 columns where
+ * they lie 900, single CTAs 900); with fewer, and with an addend, the latter. */
+static bool tc_use_ring(const TcArgs &g, long long nbatch) {
+  if (g.vec_io || g.c_bf16 || g.has_x || g.M <= TC_BM) return false;
+  const char *e = getenv("POLY_B200_TC_RING");             /* "0": never (measurements) */
+  if (e && e[0] == '0') return false;
+  return ((long long)(g.M + 2 * TC_BM - 1) / (2 * TC_BM)) * ((g.N + 255) / 256) * nbatch >= 74;
+}
+
 template <bool MN>
 static int tc_launch_16(int BN, int ctas, const CUtensorMap &ma, const CUtensorMap &mb, TcArgs &g, long long nbatch, cudaStream_t stream) {
+  if (ctas == 2 && tc_use_ring(g, nbatch)) return tc_launch<256, 2, false, false, MN, true>(ma, mb, g, nbatch, stream);
   if (ctas == 2) return tc_launch<256, 2, false, false, MN>(ma, mb, g, nbatch, stream);
   if (BN == 256) return tc_launch<256, 1, false, false, MN>(ma, mb, g, nbatch, stream);
   if (BN == 192) return tc_launch<192, 1, false, false, MN>(ma, mb, g, nbatch, stream);
@@ -1169,6 +1226,7 @@ int pb_gemm_tc_run(PbGemmProgram &p, void *const *bufs, cudaStream_t stream, int
     const long long pair_tiles = ((g.M + 2 * TC_BM - 1) / (2 * TC_BM)) * ((g.N + 255) / 256) * p.nbatch;
     const double pair_cost = (double)((pair_tiles + 73) / 74) * (0.85 * k_model * 256 + 94000.0);
     if (k_model >= 1024 && pair_tiles >= 74 && pair_cost <= best_cost && !getenv("POLY_B200_TC_BN")) { ctas = 2; BN = 256; }
+    if (!fp32x3 && pair_cost <= best_cost && tc_use_ring(g, p.nbatch) && !getenv("POLY_B200_TC_BN")) { ctas = 2; BN = 256; }
     const char *c = getenv("POLY_B200_TC_CTAS");
     if (c && atoi(c) == 1) ctas = 1;
     if (c && atoi(c) == 2) { ctas = 2; BN = 256; }

@@ -141,3 +141,17 @@ def test_f32_operands_rounded_to_bf16(kernels, m, n, k, a_kfast, b_kfast, pad): 
     assert kernels.c.poly_b200_gemm(m, n, k, kernels.put(ma), a_sm, a_sk, kernels.put(mb), b_sk, b_sn, c, n, None, 0, 0) == 0, kernels.error()
     want = bf16(a).astype(np.float64) @ bf16(b).T.astype(np.float64)
     assert_close(kernels.get(c, (m, n)), want, 1e-4, f'policy {m} {n} {k}')
+
+
+@pytest.mark.parametrize('relu', [0, 1])
+@pytest.mark.parametrize('m,n,k,pitch,offset', [(2312, 2185, 72, 2185, 0), (129, 18945, 64, 18950, 4), (2561, 1799, 1048, 1803, 12)], ids=str)
+def test_rows_written_line_by_line(kernels, m, n, k, pitch, offset, relu):  # noqa: F811
+    """CTA pairs whose result rows start anywhere: every offset of a row in its 128-byte line, parts of a tile with
+    one column and none, ragged rows; what lies between the rows stays as it was."""
+    rng = np.random.default_rng([m, n, k])
+    a, b = bf16(rng.standard_normal((m, k))), bf16(rng.standard_normal((n, k)))
+    c = kernels.put(np.full((m, pitch), 7, np.float32), offset)
+    assert kernels.c.poly_b200_gemm(m, n, k, kernels.put(bits(a)), k, 1, kernels.put(bits(b)), 1, k, c, pitch, None, relu, 1) == 0, kernels.error()
+    got, want = kernels.get(c, (m, pitch)), a.astype(np.float64) @ b.T.astype(np.float64)
+    assert np.all(got[:, n:] == 7)
+    assert_close(got[:, :n], np.maximum(want, 0) if relu else want, 1e-4, f'{m} {n} {k}')
