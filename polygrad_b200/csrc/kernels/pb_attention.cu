@@ -425,6 +425,7 @@ pb200_flash_attn2(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   const int qb = g.n_qblocks - 1 - (int)(blockIdx.x / n_bh), bh = blockIdx.x % n_bh;
   const int nkb = g.T / AT_BK;
 
+  pb_grid_wait();
   if ((int)threadIdx.x < nkb) {
     const int j = threadIdx.x;
     const float *rec = g.tile_const + (long long)AT_REC * (qb * nkb + j);
@@ -880,6 +881,7 @@ struct PrepareArgs {
   const float *mask; int nk; float *tiles; int n_mask;
 };
 __global__ void __launch_bounds__(256) pb200_attn_prepare(const PrepareArgs a) {
+  pb_grid_wait();
   if ((int)blockIdx.x < a.n_mask) { mask_tile(a.mask, a.T, 1, a.nk, a.tiles, blockIdx.x / a.nk, blockIdx.x % a.nk); return; }
   const int id = blockIdx.x - a.n_mask, blk = id % a.nblk, bh = id / a.nblk;
   /* 8 threads per row of 64, 32 rows per pass */
@@ -1103,8 +1105,8 @@ int pb_attention_launch(const PbAttnOperand &q, const PbAttnOperand &k, const Pb
   pb_tc_mark_used();
   pb_tc_configure_backoff();
   if (v1) pb200_flash_attn<<<(unsigned)grid, AT_THREADS, AT_SMEM, stream>>>(mq, mk, mv, g);
-  else pb200_flash_attn2<<<(unsigned)grid, AT_THREADS, AT2_SMEM, stream>>>(mq, mk, mv, g);
   cudaError_t e = cudaGetLastError();
+  if (!v1 && e == cudaSuccess) e = pb_launch_chained(pb200_flash_attn2, dim3((unsigned)grid), AT_THREADS, AT2_SMEM, stream, 1, mq, mk, mv, g);
   if (e != cudaSuccess) { pb_set_error("attention launch: %s", cudaGetErrorString(e)); return -1; }
   return 0;
 }
@@ -1137,11 +1139,12 @@ extern "C" int poly_b200_attention(const float *q, const float *k, const float *
     float *norms = records + AT_REC * nq * nq;
     if (attn_skips()) { a.qn = norms; a.kn = norms + BH * nq; }
     a.mask = mask; a.nk = (int)nq; a.tiles = records; a.n_mask = (int)(nq * nq);
-    pb200_attn_prepare<<<(unsigned)n_blocks, 256, 0, stream>>>(a);
+    cudaError_t e = pb_launch_chained(pb200_attn_prepare, dim3((unsigned)n_blocks), 256, 0, stream, 1, a);
     const int bext[2] = {H, B};
     const long long o_sb[2] = {(long long)T * AT_HD, (long long)H * T * AT_HD};
     PbAttnOperand oq{qb, D, {AT_HD, (long long)T * D, 0}}, ok{kb, D, {AT_HD, (long long)T * D, 0}}, ov{vb, D, {AT_HD, (long long)T * D, 0}};
-    rc = pb_attention_launch(oq, ok, ov, mask, T, 1, scale, out, false, 2, bext, o_sb, AT_HD, BH, T, stream, records, 2, a.qn);
+    if (e != cudaSuccess) pb_set_error("attention launch: %s", cudaGetErrorString(e));
+    else rc = pb_attention_launch(oq, ok, ov, mask, T, 1, scale, out, false, 2, bext, o_sb, AT_HD, BH, T, stream, records, 2, a.qn);
     if (rc == 0) pb_count_launch(true, 2);
   } else if (qb && kb && vb) {
     /* operands off the 16-byte grid: fp32 [b][t][h][d] -> bf16 in the same layout */

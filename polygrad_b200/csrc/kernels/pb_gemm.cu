@@ -378,6 +378,8 @@ __device__ __forceinline__ void stage_operand(uint32_t dst, const float *base, l
 template <bool AK, bool BKm>
 __global__ void __launch_bounds__(256, 1) pb200_sgemm_small(const SgemmArgs g, const int n_split, const bool wide_a, const bool wide_b) {
   extern __shared__ __align__(16) float sm[];
+  pb_grid_release();
+  pb_grid_wait();
   long long oa = 0, ob = 0, oc = 0, ox = 0;
   {
     int rem = blockIdx.z;
@@ -492,13 +494,7 @@ static int small_launch(const SgemmArgs &g, dim3 grid, int n_split, bool wide_a,
   static bool configured = false;
   cudaError_t e = cudaSuccess;
   if (!configured) { e = cudaFuncSetAttribute(pb200_sgemm_small<AK, BKm>, cudaFuncAttributeMaxDynamicSharedMemorySize, S_SMEM); configured = e == cudaSuccess; }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid.x * (unsigned)n_split, grid.y, grid.z); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = S_SMEM; cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)n_split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
-  if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, pb200_sgemm_small<AK, BKm>, g, n_split, wide_a, wide_b);
+  if (e == cudaSuccess) e = pb_launch_chained(pb200_sgemm_small<AK, BKm>, dim3(grid.x * (unsigned)n_split, grid.y, grid.z), 256, S_SMEM, stream, (unsigned)n_split, g, n_split, wide_a, wide_b);
   if (e != cudaSuccess) { pb_set_error("sgemm launch: %s", cudaGetErrorString(e)); return -1; }
   return 0;
 }

@@ -190,6 +190,8 @@ pb200_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
   if constexpr (CTAS == 2) cluster_sync_all();
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
+  pb_grid_release();
+  pb_grid_wait();
 
   if (warp == 0) {
     /* ── TMA producer ── */
@@ -738,18 +740,7 @@ static int tc_launch(const CUtensorMap &ma, const CUtensorMap &mb, TcArgs &g, lo
   const int units = sm_count() / CTAS;
   const int grid = (int)(tiles < units ? tiles : units) * CTAS;
   cudaError_t e;
-  if (CTAS == 1) {
-    pb200_gemm_tc<BN, CTAS, PROMOTE, TF32, MN, RING><<<grid, TC_THREADS, TcSmem<BN, CTAS, TF32, RING>::BYTES, stream>>>(ma, mb, g);
-    e = cudaGetLastError();
-  } else {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid); cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = TcSmem<BN, CTAS, TF32, RING>::BYTES; cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = CTAS; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, pb200_gemm_tc<BN, CTAS, PROMOTE, TF32, MN, RING>, ma, mb, g);
-  }
+  e = pb_launch_chained(pb200_gemm_tc<BN, CTAS, PROMOTE, TF32, MN, RING>, dim3((unsigned)grid), TC_THREADS, TcSmem<BN, CTAS, TF32, RING>::BYTES, stream, CTAS, ma, mb, g);
   if (e != cudaSuccess) { pb_set_error("tensor-core gemm launch: %s", cudaGetErrorString(e)); return -1; }
   return 0;
 }
@@ -800,6 +791,8 @@ struct Pack16 {
 struct Pack16Jobs { Pack16 job[2]; int blocks0; };
 
 __global__ void __launch_bounds__(256) pb200_pack16(const Pack16Jobs p) {
+  pb_grid_release();
+  pb_grid_wait();
   const bool second = (int)blockIdx.x >= p.blocks0;
   const Pack16 &a = p.job[second ? 1 : 0];
   const int b = second ? blockIdx.x - p.blocks0 : blockIdx.x;
@@ -936,6 +929,8 @@ struct SplitArgs {
 template <bool KFAST>
 __global__ void __launch_bounds__(256) pb200_split_tf32(const SplitArgs a) {
   __shared__ float tile[KFAST ? 1 : 64][65];       /* [k][row] */
+  pb_grid_release();
+  pb_grid_wait();
   const int t = blockIdx.x % (a.tr * a.tk), z = blockIdx.x / (a.tr * a.tk);
   const int r0 = (t / a.tk) * 64, k0 = (t % a.tk) * 64;
   long long rem = z, o = 0;
@@ -1034,9 +1029,7 @@ static const void *tc_operand_x3(PbGemmProgram &p, PbTcOperand &cache, const voi
   const long long blocks = (long long)a.tr * a.tk * nz;
   if (blocks > 2147483647LL) { pb_set_error("gemm: operand too large to split"); ok = false; }
   if (ok) {
-    if (in_place && !kfast) pb200_split_tf32<false><<<(unsigned)blocks, 256, 0, stream>>>(a);
-    else pb200_split_tf32<true><<<(unsigned)blocks, 256, 0, stream>>>(a);
-    ok = cudaGetLastError() == cudaSuccess;
+    ok = pb_launch_chained(in_place && !kfast ? pb200_split_tf32<false> : pb200_split_tf32<true>, dim3((unsigned)blocks), 256, 0, stream, 1, a) == cudaSuccess;
     p.launches++;
   }
   pb_scratch_free(dense);           /* stream-ordered pool: reusable by later work on this stream */
@@ -1136,8 +1129,7 @@ int pb_gemm_tc_run(PbGemmProgram &p, void *const *bufs, cudaStream_t stream, int
       if (ok) {
         jobs.blocks0 = (jobs.job[0].total + 511) / 512;
         const int blocks = jobs.blocks0 + (n_jobs == 2 ? (jobs.job[1].total + 511) / 512 : 0);
-        pb200_pack16<<<(unsigned)blocks, 256, 0, stream>>>(jobs);
-        const cudaError_t e = cudaGetLastError();
+        const cudaError_t e = pb_launch_chained(pb200_pack16, dim3((unsigned)blocks), 256, 0, stream, 1, jobs);
         ok = e == cudaSuccess;
         if (!ok) pb_set_error("gemm: operand copy launch: %s", cudaGetErrorString(e));
         p.launches++;

@@ -1,0 +1,55 @@
+"""Launches that may start while their predecessors drain, captured into a graph between work of other kinds:
+the replays give what the calls gave."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from kernel_lib import kernels  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+def test_captured_chain(kernels):  # noqa: F811
+    c, P = kernels.c, ctypes.c_void_p
+    c.poly_b200_capture_end.restype, c.poly_b200_capture_end.argtypes = P, [ctypes.c_int]
+    c.poly_b200_graph_launch.argtypes = [P, ctypes.c_ulonglong, ctypes.c_ulonglong]
+    c.poly_b200_graph_destroy.restype, c.poly_b200_graph_destroy.argtypes = None, [P]
+    c.poly_cuda_memset.argtypes = [ctypes.c_ulonglong, ctypes.c_ubyte, ctypes.c_size_t]
+    rng = np.random.default_rng(3)
+    n = 256
+    x = [rng.standard_normal((n, n)).astype(np.float32) / 16 for _ in range(3)]
+    a, b, d = (kernels.put(v) for v in x)
+    t, u, w = (kernels.put(np.zeros((n, n), np.float32)) for _ in range(3))
+    q = kernels.put(rng.standard_normal((1, 128, 2, 64)).astype(np.float32))
+    mask, o = kernels.put(np.zeros((128, 128), np.float32)), kernels.put(np.zeros((1, 2, 128, 64), np.float32))
+
+    def chain():
+        # every call reads what the one before it wrote
+        c.poly_b200_set_gemm_policy(0)
+        rc = [c.poly_b200_gemm(n, n, n, a, n, 1, b, n, 1, t, n, None, 0, 0), c.poly_b200_gemm(n, n, n, t, n, 1, d, n, 1, u, n, None, 0, 0)]
+        c.poly_b200_set_gemm_policy(1)
+        rc.append(c.poly_b200_gemm(n, n, n, u, n, 1, d, n, 1, w, n, None, 0, 0))
+        rc.append(c.poly_cuda_memset(t, 1, n * n * 4))
+        rc.append(c.poly_b200_gemm(n, n, n, w, 1, n, t, n, 1, u, n, None, 0, 0))
+        rc.append(c.poly_b200_attention(q, u, w, mask, 0.125, o, 1, 2, 128))
+        assert not any(rc), kernels.error()
+
+    def results():
+        return [kernels.get(p, s).copy() for p, s in ((t, (n, n)), (u, (n, n)), (w, (n, n)), (o, (1, 2, 128, 64)))]
+
+    for _ in range(3):
+        chain()
+    want = results()
+    assert c.poly_b200_capture_begin() == 0
+    chain()
+    graph = c.poly_b200_capture_end(0)
+    assert graph, kernels.error()
+    for p in (u, w):
+        c.poly_cuda_memset(p, 2, n * n * 4)
+    for _ in range(3):
+        assert c.poly_b200_graph_launch(graph, 0, 0) == 0, kernels.error()
+    got = results()
+    c.poly_b200_graph_destroy(graph)
+    for g, v in zip(got, want):
+        assert np.array_equal(g.view(np.uint32), v.view(np.uint32))
