@@ -346,7 +346,7 @@ static SgemmFn pick_vec(bool va, bool vb) {
  * bound), and four k slabs of 32 are in flight (cp.async, zero-filled past every edge).  Partial sums
  * are added in a fixed order: groups in shared memory, then the CTAs of a cluster over distributed shared memory.
  * 32 x 32 tiles with 2 x 2 results and one slab in flight: 256 x 512 x 784 28.7 us, 256 x 10 x 512 19.1 us;
- * 18.1 and 10.2 like this. */
+ * 14.8 and 8.1 like this, launched behind other work. */
 #define SB 64
 #define SK 32
 #define S_STAGES 4
@@ -409,11 +409,11 @@ __global__ void __launch_bounds__(256, 1) pb200_sgemm_small(const SgemmArgs g, c
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  float acc[8][8];
+  float2 acc[8][4];                                          /* [row][pair of columns]: two multiply-adds per instruction */
 #pragma unroll
   for (int i = 0; i < 8; i++)
 #pragma unroll
-    for (int j = 0; j < 8; j++) acc[i][j] = 0.0f;
+    for (int j = 0; j < 4; j++) acc[i][j] = make_float2(0.0f, 0.0f);
 #pragma unroll
   for (int s = 0; s < S_STAGES - 1; s++) fetch(s);
   for (int s = 0; s < n_slabs; s++) {
@@ -439,7 +439,8 @@ __global__ void __launch_bounds__(256, 1) pb200_sgemm_small(const SgemmArgs g, c
 #pragma unroll
         for (int i = 0; i < 8; i++)
 #pragma unroll
-          for (int j = 0; j < 8; j++) acc[i][j] = fmaf(a[i][kk], b[j][kk], acc[i][j]);
+          for (int j = 0; j < 4; j++)
+            acc[i][j] = __ffma2_rn(make_float2(a[i][kk], a[i][kk]), make_float2(b[2 * j][kk], b[2 * j + 1][kk]), acc[i][j]);
     }
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
@@ -447,7 +448,7 @@ __global__ void __launch_bounds__(256, 1) pb200_sgemm_small(const SgemmArgs g, c
 #pragma unroll
   for (int i = 0; i < 8; i++)
 #pragma unroll
-    for (int j = 0; j < 8; j++) sm[(group * SB + row_of(i)) * S_PITCH + col_of(j)] = acc[i][j];
+    for (int j = 0; j < 8; j++) sm[(group * SB + row_of(i)) * S_PITCH + col_of(j)] = j & 1 ? acc[i][j >> 1].y : acc[i][j >> 1].x;
   __syncthreads();
 
   float *__restrict__ C = g.C + oc;
