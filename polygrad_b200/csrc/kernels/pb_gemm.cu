@@ -11,8 +11,8 @@
  *      [B, T, H*hd] from [B, H, T, hd] storage) is packed into a dense scratch
  *      matrix by a strided copy first;
  *   3. launches the fp32 CUDA-core kernel, or -- for bf16 operands or under the
- *      bf16 compute policy (POLY_B200_GEMM=bf16) -- converts both operands to
- *      K-major bf16 (weights once, cached per buffer version) and runs the
+ *      bf16 compute policy (POLY_B200_GEMM=bf16) -- copies operands that cannot be
+ *      read in place to bf16 (weights once, cached per buffer version) and runs the
  *      tcgen05 tensor-core kernel (pb_gemm_tc.cu).
  *
  * fp32 kernel: 128x128 block tile, 16-deep k slices, 256 threads, 8x8 register
@@ -609,7 +609,7 @@ int PbGemmProgram::launch(void *const *bufs, cudaStream_t stream) {
     if (dtype != PB_F32 || a_bf16 || c_bf16) { pb_set_error("gemm: 16-bit operands need the tensor-core kernel, which rejected this shape"); return -1; }
   }
   /* float32 contractions of at least 2^30 multiply-adds run on the tensor cores as three tf32
-   * products, the partial sums of every eight k-blocks added up in registers (float32-accurate:
+   * products, the partial sums of every two k-blocks added up in registers (float32-accurate:
    * the 1e-5 bound of this path holds at every K; a scale factor is applied to the sum before the
    * addend).  Small ones stay on the CUDA-core kernels.  POLY_B200_FP32=simt keeps everything there; =tcp sends every shape the tensor-core
    * kernel accepts; =tc sums the whole k axis in tensor memory instead, whose accumulation

@@ -3,7 +3,8 @@
  * cores (tcgen05), operands staged by TMA, accumulators in tensor memory.
  *
  * Problem: C[b, m, n] = sum_k A[b, m, k] * B[b, n, k] (+ X) (relu), A and B
- * bfloat16 with k contiguous ("K-major"), C float32 row-major.
+ * bfloat16 with k contiguous ("K-major") or with their rows contiguous (template
+ * parameter MN), C float32 or bfloat16, row-major.
  * polygrad produces this either from bf16 buffers cast to float before the MUL,
  * or -- under POLY_B200_GEMM=bf16 -- from fp32 buffers whose values are rounded
  * to bf16 (nearest even) on the way in; products and sums stay fp32.
@@ -24,8 +25,8 @@
  * Two accumulator buffers in tensor memory let the MMA warp start the next tile
  * while the epilogue drains the previous one.
  *
- * For long K the same kernel runs as CTA pairs (template parameter CTAS = 2, a
- * cluster of two CTAs on neighbouring SMs): tcgen05.mma.cta_group::2 with M =
+ * For long K, and for large results with unaligned rows (RING: written line by
+ * line), the same kernel runs as CTA pairs (template parameter CTAS = 2, a cluster of two CTAs on neighbouring SMs): tcgen05.mma.cta_group::2 with M =
  * 256 computes a 256 x 256 tile, 128 rows in each CTA's tensor memory; each CTA
  * stages its own 128 rows of A and one half of the tile's B rows (the tensor
  * cores read both halves), so a stage is 32 KB instead of 48 and six fit.  The
