@@ -622,13 +622,22 @@ int PbGemmProgram::launch(void *const *bufs, cudaStream_t stream) {
      * cost more than they save: with the threshold at 2^26 the MLP forward went from 44.6 to 52.8 us
      * and a small training step from 3.85 to 4.27 ms (and a single 2^28 contraction in that step cost
      * 0.3 ms), so the threshold is 2^30 multiply-adds, 1024^3 */
-    if (!m) mode = (double)M * (double)N * (double)K * (double)nbatch >= 1073741824.0 ? 2 : 0;
+    const double work = (double)M * (double)N * (double)K * (double)nbatch;
+    if (!m && work >= 1073741824.0) mode = 2;
+    /* From half of that on, where half the SMs get a 128 x 64 tile, every k-block is a partial sum of its own: no less accurate
+     * than the CUDA cores' sums and faster (us, rms error against float64: 1024 x 1024 x 900 81, 2.7e-7 there, 40,
+     * 1.6e-7 here; 8192 x 512 x 128 33, 2.0e-7 and 22, 1.4e-7; 3000 x 1000 x 300 70, 3.1e-7 and 33, 1.4e-7;
+     * 4096 x 4096 x 60 66, 1.40e-7 and 39, 1.33e-7).  With fewer tiles the split k axis wins (512 x 512 x 3000: 67 and 93). */
+    else if (!m && work >= 536870912.0 && K >= 32 && (double)((M + 127) / 128) * (double)((N + 63) / 64) * (double)nbatch >= 74) mode = 3;
+    else if (!m) mode = 0;
     else if (strcmp(m, "tc") == 0) mode = 1;
     else if (strcmp(m, "tcp") == 0) mode = 2;
     if (alpha != 1.0f && mode == 1) mode = 0;          /* a scaled sum: the promoted kernels or the CUDA cores */
     if (mode) {
       int rc = pb_gemm_tc_run(*this, bufs, stream, mode);
-      if (rc != PB_TC_UNSUPPORTED) return rc;
+      /* (below 2^30 a full pool sends the call to the CUDA cores, which need none) */
+      if (rc == PB_TC_NO_SCRATCH && mode != 3) rc = -1;
+      if (rc != PB_TC_UNSUPPORTED && rc != PB_TC_NO_SCRATCH) return rc;
     }
   }
   SgemmArgs g{};

@@ -12,6 +12,7 @@
 enum { PB_F32 = 0, PB_BF16 = 1, PB_F16 = 2 };      /* storage type of a contraction's operands */
 #define PB_PACK_MAX_AXES 12
 #define PB_TC_UNSUPPORTED 77
+#define PB_TC_NO_SCRATCH 78      /* float32 modes: the operands' parts did not fit the pool; nothing was computed */
 
 /* A launch that may start while the work before it on the stream drains (programmatic dependence): its blocks set up
  * barriers and tensor memory and then wait in pb_grid_wait() for all of that work, results included, before they
@@ -103,7 +104,7 @@ bool pb_gemm_tc_static_ok(const PbGemmProgram &p);
 
 /* Tensor-core path: returns 0 / -1, or PB_TC_UNSUPPORTED when the shape is not handled. */
 /* fp32_mode 0: 16-bit operands.  1: float32 operands as three tf32 products, summed in tensor memory.
- * 2: the same with the partial sums moved to registers every few k-blocks (float32-accurate). */
+ * 2: the same with the partial sums moved to registers every two k-blocks (float32-accurate), 3: every block. */
 int pb_gemm_tc_run(PbGemmProgram &p, void *const *bufs, cudaStream_t stream, int fp32_mode = 0);
 
 /* The tensor-core kernel on ready-made bfloat16 K-major operands; touches no

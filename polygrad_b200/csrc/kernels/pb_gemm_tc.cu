@@ -1093,7 +1093,7 @@ bool pb_gemm_tc_static_ok(const PbGemmProgram &p) {
 }
 
 int pb_gemm_tc_run(PbGemmProgram &p, void *const *bufs, cudaStream_t stream, int fp32_mode) {
-  const bool fp32x3 = fp32_mode != 0, promote = fp32_mode == 2;
+  const bool fp32x3 = fp32_mode != 0, promote = fp32_mode >= 2;
   /* output must be a row-major (or column-major: swap roles) matrix per batch entry */
   bool swap = false;
   if (p.c_sn != 1 || p.N == 1) { if (p.c_sm == 1 && p.M > 1) swap = true; else if (p.c_sn != 1) return PB_TC_UNSUPPORTED; }
@@ -1144,7 +1144,7 @@ int pb_gemm_tc_run(PbGemmProgram &p, void *const *bufs, cudaStream_t stream, int
       }
     }
   }
-  if (!va.ptr || !vb.ptr) { pb_scratch_free(scr_a); pb_scratch_free(scr_b); return -1; }
+  if (!va.ptr || !vb.ptr) { pb_scratch_free(scr_a); pb_scratch_free(scr_b); return fp32x3 ? PB_TC_NO_SCRATCH : -1; }
 
   TcArgs g{};
   long long rowsA = p.M, rowsB = p.N;
@@ -1240,7 +1240,7 @@ int pb_gemm_tc_run(PbGemmProgram &p, void *const *bufs, cudaStream_t stream, int
      * 4.7e-7, 157 us; 4 blocks 8.2e-7 to 8.5e-7, 149 us (256 elements of one 3K axis, as it was: 6.4e-7 to
      * 7.1e-7, 244 us); POLY_B200_TC_KCHUNK overrides (measurements) */
     const char *kc = getenv("POLY_B200_TC_KCHUNK");
-    g.kchunk = kc && atoi(kc) > 0 ? atoi(kc) : 2;
+    g.kchunk = kc && atoi(kc) > 0 ? atoi(kc) : fp32_mode == 3 ? 1 : 2;
     if (ctas == 2) rc = tc_launch<256, 2, true, true>(ma, mb, g, p.nbatch, stream);
     else rc = BN == 128 ? tc_launch<128, 1, true, true>(ma, mb, g, p.nbatch, stream) : tc_launch<64, 1, true, true>(ma, mb, g, p.nbatch, stream);
   } else if (fp32x3) {

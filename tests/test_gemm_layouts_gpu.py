@@ -155,3 +155,18 @@ def test_rows_written_line_by_line(kernels, m, n, k, pitch, offset, relu):  # no
     got, want = kernels.get(c, (m, pitch)), a.astype(np.float64) @ b.T.astype(np.float64)
     assert np.all(got[:, n:] == 7)
     assert_close(got[:, :n], np.maximum(want, 0) if relu else want, 1e-4, f'{m} {n} {k}')
+
+
+@pytest.mark.parametrize('a_kfast,b_kfast', [(True, False), (False, True)])
+@pytest.mark.parametrize('m,n,k', [(1024, 1024, 512), (1023, 1025, 513), (100, 12321, 438), (4096, 4100, 33), (512, 512, 2050)], ids=str)
+def test_f32_default_route_around_half_a_giga(kernels, m, n, k, a_kfast, b_kfast):  # noqa: F811
+    """2^29 multiply-adds, a little more and a little less, many and few tiles: no less accurate than sums of float32."""
+    rng = np.random.default_rng([m, n, k])
+    a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
+    ma, (a_sm, a_sk) = stored(a, a_kfast, 0, rng, lambda x: x)
+    mb, (b_sn, b_sk) = stored(b, b_kfast, 0, rng, lambda x: x)
+    c = kernels.put(np.zeros((m, n), np.float32))
+    assert kernels.c.poly_b200_gemm(m, n, k, kernels.put(ma), a_sm, a_sk, kernels.put(mb), b_sk, b_sn, c, n, None, 0, 0) == 0, kernels.error()
+    got, want = kernels.get(c, (m, n)), a.astype(np.float64) @ b.T.astype(np.float64)
+    assert_close(got, want, 1e-5, f'f32 {m} {n} {k}')
+    assert np.sqrt(np.mean((got - want) ** 2)) <= 6e-7 * np.sqrt(np.mean(want ** 2))      # sequential float32 sums: 6e-7 at these K
