@@ -46,9 +46,11 @@ int pb_pack_launch(const void *src, void *dst, int naxes, const long long *ext, 
  * the output C, in A, in B and in the addend X (0 where it does not appear). */
 struct PbGemmAxis { char kind; long long ext, sc, sa, sb, sx; };
 
-/* A bf16, K-major copy of one operand, kept while the source is unchanged. */
+/* A copy of one operand for the tensor cores, kept while the source is unchanged.  form: what `data` holds, 16-bit
+ * elements or the two tf32 parts of float32 ones (one program makes either, as the policy says at the call). */
+enum { PB_TC_FORM_16 = 1, PB_TC_FORM_TF32 = 2 };
 struct PbTcOperand {
-  void *data = nullptr; size_t bytes = 0;
+  void *data = nullptr; size_t bytes = 0; int form = 0;
   const void *src = nullptr; uint64_t version = 0;
   int misses = 0;      /* conversions done; an operand that changes every call stops being cached */
 };

@@ -849,7 +849,7 @@ static int tc_operand(PbGemmProgram &p, PbTcOperand &cache, const void *src_buf,
   v->pitch = plain ? lp : Kp; v->bpitch = plain ? lines * lp : rows * Kp;
   const size_t bytes = (size_t)(p.nbatch * v->bpitch) * 2;
   const uint64_t ver = pb_buffer_version(src_buf);
-  if (cache.data && cache.src == src_buf && cache.version == ver && cache.bytes == bytes && ver != 0) { v->ptr = cache.data; return 0; }
+  if (cache.data && cache.form == PB_TC_FORM_16 && cache.src == src_buf && cache.version == ver && cache.bytes == bytes && ver != 0) { v->ptr = cache.data; return 0; }
   const bool transient = cache.misses >= 2 || ver == 0;
   void *dst;
   if (transient) {
@@ -862,7 +862,7 @@ static int tc_operand(PbGemmProgram &p, PbTcOperand &cache, const void *src_buf,
     if (!cache.data) { cache.data = pb_scratch_alloc(bytes); cache.bytes = bytes; }
     if (!cache.data) return -1;
     dst = cache.data;
-    cache.src = src_buf; cache.version = ver; cache.misses++;
+    cache.form = PB_TC_FORM_16; cache.src = src_buf; cache.version = ver; cache.misses++;
   }
   if (plain) {
     const int esz = p.dtype == PB_F32 ? 4 : 2;
@@ -983,7 +983,7 @@ static const void *tc_operand_x3(PbGemmProgram &p, PbTcOperand &cache, const voi
   *scratch = nullptr;
   const size_t bytes = (size_t)(p.nbatch * rows * 2 * Kp) * 4;
   const uint64_t ver = pb_buffer_version(src_buf);
-  if (cache.data && cache.src == src_buf && cache.version == ver && cache.bytes == bytes && ver != 0) return cache.data;
+  if (cache.data && cache.form == PB_TC_FORM_TF32 && cache.src == src_buf && cache.version == ver && cache.bytes == bytes && ver != 0) return cache.data;
   const bool transient = cache.misses >= 2 || ver == 0;
   void *dst;
   if (transient) {
@@ -996,7 +996,7 @@ static const void *tc_operand_x3(PbGemmProgram &p, PbTcOperand &cache, const voi
     if (!cache.data) { cache.data = pb_scratch_alloc(bytes); cache.bytes = bytes; }
     if (!cache.data) return nullptr;
     dst = cache.data;
-    cache.src = src_buf; cache.version = ver; cache.misses++;
+    cache.form = PB_TC_FORM_TF32; cache.src = src_buf; cache.version = ver; cache.misses++;
   }
   /* an operand whose strides nest and whose k or row axis is contiguous (an activation as the model stores it;
    * a weight; the activations a weight gradient reads transposed, whose token axes nest into one k axis) is

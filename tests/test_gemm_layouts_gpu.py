@@ -170,3 +170,21 @@ def test_f32_default_route_around_half_a_giga(kernels, m, n, k, a_kfast, b_kfast
     got, want = kernels.get(c, (m, n)), a.astype(np.float64) @ b.T.astype(np.float64)
     assert_close(got, want, 1e-5, f'f32 {m} {n} {k}')
     assert np.sqrt(np.mean((got - want) ** 2)) <= 6e-7 * np.sqrt(np.mean(want ** 2))      # sequential float32 sums: 6e-7 at these K
+
+
+@pytest.mark.parametrize('first', [0, 1])
+@pytest.mark.parametrize('m,n,k', [(128, 2, 64), (2, 128, 64)], ids=str)
+def test_policy_switched_on_the_same_operands(kernels, monkeypatch, m, n, k, first):  # noqa: F811
+    """One call's operands under either policy in turn, unwritten in between: with two rows stored rows fastest, the kept
+    copies for the two policies are equally large."""
+    monkeypatch.setenv('POLY_B200_FP32', 'tcp')
+    rng = np.random.default_rng([m, n, k])
+    a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
+    ma, (a_sm, a_sk) = stored(a, m > 2, 0, rng, lambda x: x)
+    mb, (b_sn, b_sk) = stored(b, n > 2, 0, rng, lambda x: x)
+    d_a, d_b, c = kernels.put(ma), kernels.put(mb), kernels.put(np.zeros((m, n), np.float32))
+    exact = [x.astype(np.float64) @ y.T.astype(np.float64) for x, y in ((a, b), (bf16(a), bf16(b)))]
+    for policy in (first, 1 - first, first, 1 - first):
+        kernels.c.poly_b200_set_gemm_policy(policy)
+        assert kernels.c.poly_b200_gemm(m, n, k, d_a, a_sm, a_sk, d_b, b_sk, b_sn, c, n, None, 0, 0) == 0, kernels.error()
+        assert_close(kernels.get(c, (m, n)), exact[policy], 1e-5, f'policy {policy}')
