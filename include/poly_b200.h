@@ -87,10 +87,11 @@ int  poly_b200_set_device(int device);
 int  poly_b200_device(void);
 
 /* Arithmetic of fp32 contractions (polygrad matmuls on float32 buffers):
- *   0  float32 arithmetic (default): contractions of at least 2^30 multiply-adds
- *      run on the tensor cores as three tf32 products per multiply (a = hi + lo,
+ *   0  float32 arithmetic (default): contractions of at least 2^30 multiply-adds,
+ *      and of 2^29 with K >= 192 and at least 74 result tiles of 128 x 64, run on
+ *      the tensor cores as three tf32 products per multiply (a = hi + lo,
  *      hi.hi + hi.lo + lo.hi) with the partial sums added up in float32
- *      registers, within 1e-5 of the CPU at every K; smaller ones are fp32 FMAs
+ *      registers, within 1e-5 of the CPU at every K; the others are fp32 FMAs
  *      on the CUDA cores.  POLY_B200_FP32=simt|tcp|tc forces a route (tc: the
  *      sums stay in tensor memory, error about 1e-8 * K of the result's rms);
  *   1  operands rounded to bfloat16 (nearest even), products and sums in fp32,

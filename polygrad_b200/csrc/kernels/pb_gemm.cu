@@ -608,27 +608,27 @@ int PbGemmProgram::launch(void *const *bufs, cudaStream_t stream) {
     if (rc != PB_TC_UNSUPPORTED) return rc;
     if (dtype != PB_F32 || a_bf16 || c_bf16) { pb_set_error("gemm: 16-bit operands need the tensor-core kernel, which rejected this shape"); return -1; }
   }
-  /* float32 contractions of at least 2^30 multiply-adds run on the tensor cores as three tf32
-   * products, the partial sums of every two k-blocks added up in registers (float32-accurate:
-   * the 1e-5 bound of this path holds at every K; a scale factor is applied to the sum before the
-   * addend).  Small ones stay on the CUDA-core kernels.  POLY_B200_FP32=simt keeps everything there; =tcp sends every shape the tensor-core
+  /* float32 contractions run on the tensor cores as three tf32 products from 2^30 multiply-adds on, the partial sums of
+   * every two k-blocks added up in registers (the 1e-5 bound of this path holds at every K; a scale factor is applied to
+   * the sum before the addend), and, where that is at least as accurate as the CUDA cores' sums in k order, from 2^29
+   * on.  Smaller ones stay on the CUDA-core kernels.  POLY_B200_FP32=simt keeps everything there; =tcp sends every shape the tensor-core
    * kernel accepts; =tc sums the whole k axis in tensor memory instead, whose accumulation
    * truncates (error about 1e-8 * K of the result's rms; a few percent faster). */
   {
     const char *m = getenv("POLY_B200_FP32");
     int mode = 0;
-    /* back-to-back calls favour this route from far smaller sizes (256 x 784 x 512: 26.6 us on the CUDA
-     * cores, 20.6 us here), but inside a short dependent chain its extra launch and longer start-up
-     * cost more than they save: with the threshold at 2^26 the MLP forward went from 44.6 to 52.8 us
-     * and a small training step from 3.85 to 4.27 ms (and a single 2^28 contraction in that step cost
-     * 0.3 ms), so the threshold is 2^30 multiply-adds, 1024^3 */
     const double work = (double)M * (double)N * (double)K * (double)nbatch;
     if (!m && work >= 1073741824.0) mode = 2;
-    /* From half of that on, where half the SMs get a 128 x 64 tile, every k-block is a partial sum of its own: no less accurate
-     * than the CUDA cores' sums and faster (us, rms error against float64: 1024 x 1024 x 900 81, 2.7e-7 there, 40,
-     * 1.6e-7 here; 8192 x 512 x 128 33, 2.0e-7 and 22, 1.4e-7; 3000 x 1000 x 300 70, 3.1e-7 and 33, 1.4e-7;
-     * 4096 x 4096 x 60 66, 1.40e-7 and 39, 1.33e-7).  With fewer tiles the split k axis wins (512 x 512 x 3000: 67 and 93). */
-    else if (!m && work >= 536870912.0 && K >= 32 && (double)((M + 127) / 128) * (double)((N + 63) / 64) * (double)nbatch >= 74) mode = 3;
+    /* From 2^29 on every k-block is a partial sum of its own, and the error hardly depends on K, where that of sums in k
+     * order grows with its root.  rms error of the result's rms against float64, k order -> here, at K = 64, 128, 192, 512:
+     *   N(0, 1)                      1.44 -> 1.32  2.03 -> 1.35  2.48 -> 1.38  4.05 -> 1.50  (all e-7)
+     *   max(N(0, 1), 0) x |N(0, 1)|  0.87 -> 1.09  1.22 -> 1.08  1.42 -> 1.08  2.46 -> 1.17
+     *   probabilities x U(0.5, 1.5)  1.21 -> 1.82  1.66 -> 1.85  2.00 -> 1.84  3.17 -> 1.89
+     * so K >= 192.  (The tensor cores truncate: with operands of one sign all of it lies on one side, a mean error of
+     * 1.2e-7 to 1.8e-7 towards zero, where roundings in k order have none.)  And where half the SMs get a 128 x 64 tile: 1024 x 1024
+     * x 900 81 us on the CUDA cores, 40 here; 3000 x 1000 x 300 70 and 33; with fewer tiles the split k axis wins (512 x 512 x 3000:
+     * 67 and 93).  Below 2^29 the second launch and the longer start-up cost more than they save in a chain of dependent calls. */
+    else if (!m && work >= 536870912.0 && K >= 192 && (double)((M + 127) / 128) * (double)((N + 63) / 64) * (double)nbatch >= 74) mode = 3;
     else if (!m) mode = 0;
     else if (strcmp(m, "tc") == 0) mode = 1;
     else if (strcmp(m, "tcp") == 0) mode = 2;

@@ -160,7 +160,7 @@ def test_rows_written_line_by_line(kernels, m, n, k, pitch, offset, relu):  # no
 @pytest.mark.parametrize('a_kfast,b_kfast', [(True, False), (False, True)])
 @pytest.mark.parametrize('m,n,k', [(1024, 1024, 512), (1023, 1025, 513), (100, 12321, 438), (4096, 4100, 33), (512, 512, 2050)], ids=str)
 def test_f32_default_route_around_half_a_giga(kernels, m, n, k, a_kfast, b_kfast):  # noqa: F811
-    """2^29 multiply-adds, a little more and a little less, many and few tiles: no less accurate than sums of float32."""
+    """2^29 multiply-adds, a little more and a little less, many and few tiles, both routes."""
     rng = np.random.default_rng([m, n, k])
     a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
     ma, (a_sm, a_sk) = stored(a, a_kfast, 0, rng, lambda x: x)
@@ -188,3 +188,29 @@ def test_policy_switched_on_the_same_operands(kernels, monkeypatch, m, n, k, fir
         kernels.c.poly_b200_set_gemm_policy(policy)
         assert kernels.c.poly_b200_gemm(m, n, k, d_a, a_sm, a_sk, d_b, b_sk, b_sn, c, n, None, 0, 0) == 0, kernels.error()
         assert_close(kernels.get(c, (m, n)), exact[policy], 1e-5, f'policy {policy}')
+
+
+@pytest.mark.parametrize('values', ['normal', 'relu', 'positive', 'probabilities'])
+@pytest.mark.parametrize('m,n,k', [(4096, 4100, 33), (3000, 2900, 64), (2300, 2300, 112), (2048, 1600, 191), (1700, 1700, 192), (1024, 1024, 768)], ids=str)
+def test_f32_default_route_errs_no_more_than_sums_in_k_order(kernels, m, n, k, values):  # noqa: F811
+    """Around 2^29 multiply-adds, operands of either and of one sign: on a sample of the result the error is that of one
+    rounded multiply-add after the other, or less (the tenth is the sample's own scatter)."""
+    rng = np.random.default_rng([m, k])
+    a, b = rng.standard_normal((m, k)), rng.standard_normal((n, k))
+    if values == 'relu':
+        a = np.maximum(a, 0)
+    elif values == 'positive':
+        a, b = rng.random((m, k)), rng.random((n, k))
+    elif values == 'probabilities':
+        a = np.exp(2 * a)
+        a, b = a / a.sum(1, keepdims=True), rng.random((n, k)) + 0.5
+    a, b = a.astype(np.float32), b.astype(np.float32)
+    c = kernels.put(np.zeros((m, n), np.float32))
+    assert kernels.c.poly_b200_gemm(m, n, k, kernels.put(a), k, 1, kernels.put(b.T), n, 1, c, n, None, 0, 0) == 0, kernels.error()
+    rows, cols = rng.permutation(m)[:96], rng.permutation(n)[:96]
+    x, y = a[rows].astype(np.float64), b[cols].astype(np.float64)
+    acc = np.zeros((96, 96), np.float32)
+    for i in range(k):
+        acc = (acc + np.outer(x[:, i], y[:, i])).astype(np.float32)
+    err = [np.sqrt(np.mean((v - x @ y.T) ** 2)) for v in (kernels.get(c, (m, n))[np.ix_(rows, cols)], acc)]
+    assert err[0] <= 1.1 * err[1]
