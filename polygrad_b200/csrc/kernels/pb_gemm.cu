@@ -627,15 +627,17 @@ int PbGemmProgram::launch(void *const *bufs, cudaStream_t stream) {
      * so K >= 192.  (The tensor cores truncate: with operands of one sign all of it lies on one side, a mean error of
      * 1.2e-7 to 1.8e-7 towards zero, where roundings in k order have none.)  And where half the SMs get a 128 x 64 tile: 1024 x 1024
      * x 900 81 us on the CUDA cores, 40 here; 3000 x 1000 x 300 70 and 33; with fewer tiles the split k axis wins (512 x 512 x 3000:
-     * 67 and 93).  Below 2^29 the second launch and the longer start-up cost more than they save in a chain of dependent calls. */
-    else if (!m && work >= 536870912.0 && K >= 192 && (double)((M + 127) / 128) * (double)((N + 63) / 64) * (double)nbatch >= 74) mode = 3;
+     * 67 and 93).  Below 2^29 the second launch and the longer start-up cost more than they save in a chain of dependent calls.  Not in a
+     * capture of the caller's: there the CUDA cores read the operands as they are at each replay, and need no memory. */
+    else if (!m && work >= 536870912.0 && K >= 192 && (double)((M + 127) / 128) * (double)((N + 63) / 64) * (double)nbatch >= 74 &&
+             !pb_captured_by_caller()) mode = 3;
     else if (!m) mode = 0;
     else if (strcmp(m, "tc") == 0) mode = 1;
     else if (strcmp(m, "tcp") == 0) mode = 2;
     if (alpha != 1.0f && mode == 1) mode = 0;          /* a scaled sum: the promoted kernels or the CUDA cores */
     if (mode) {
       int rc = pb_gemm_tc_run(*this, bufs, stream, mode);
-      /* (below 2^30 a full pool sends the call to the CUDA cores, which need none) */
+      /* (below 2^30 a pool without memory for the parts sends the call to the CUDA cores) */
       if (rc == PB_TC_NO_SCRATCH && mode != 3) rc = -1;
       if (rc != PB_TC_UNSUPPORTED && rc != PB_TC_NO_SCRATCH) return rc;
     }

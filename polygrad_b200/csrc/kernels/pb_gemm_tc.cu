@@ -977,9 +977,11 @@ __global__ void __launch_bounds__(256) pb200_split_tf32(const SplitArgs a) {
   }
 }
 
-/* The two parts of A or B, [2][nbatch][rows][Kp] float32; cached like the bf16 copies. */
+/* The two parts of A or B, [2][nbatch][rows][Kp] float32; cached like the bf16 copies.  optional: the caller has another
+ * way when the pool has no memory for them. */
 static const void *tc_operand_x3(PbGemmProgram &p, PbTcOperand &cache, const void *src_buf, long long off, bool is_a,
-                                 long long rows, long long Kp, cudaStream_t stream, void **scratch) {
+                                 long long rows, long long Kp, bool optional, cudaStream_t stream, void **scratch) {
+  void *(*const take)(size_t) = optional ? pb_scratch_try : pb_scratch_alloc;
   *scratch = nullptr;
   const size_t bytes = (size_t)(p.nbatch * rows * 2 * Kp) * 4;
   const uint64_t ver = pb_buffer_version(src_buf);
@@ -988,12 +990,12 @@ static const void *tc_operand_x3(PbGemmProgram &p, PbTcOperand &cache, const voi
   void *dst;
   if (transient) {
     if (cache.data) { pb_scratch_free(cache.data); cache.data = nullptr; cache.bytes = 0; }
-    dst = pb_scratch_alloc(bytes);
+    dst = take(bytes);
     if (!dst) return nullptr;
     *scratch = dst;
   } else {
     if (cache.data && cache.bytes != bytes) { pb_scratch_free(cache.data); cache.data = nullptr; }
-    if (!cache.data) { cache.data = pb_scratch_alloc(bytes); cache.bytes = bytes; }
+    if (!cache.data) { cache.data = take(bytes); cache.bytes = bytes; }
     if (!cache.data) return nullptr;
     dst = cache.data;
     cache.form = PB_TC_FORM_TF32; cache.src = src_buf; cache.version = ver; cache.misses++;
@@ -1020,7 +1022,7 @@ static const void *tc_operand_x3(PbGemmProgram &p, PbTcOperand &cache, const voi
     for (auto &b : p.b_ax) { a.ext[a.naxes] = (int)b.ext; a.sstride[a.naxes++] = sel(b); }
   } else {
     if (p.nbatch * rows > 2147483647LL - 64) ok = false;
-    dense = ok ? pb_scratch_alloc((size_t)(p.nbatch * rows * Kp) * 4) : nullptr;
+    dense = ok ? take((size_t)(p.nbatch * rows * Kp) * 4) : nullptr;
     ok = dense != nullptr && p.pack_into(dense, src_buf, off, is_a, PB_F32, PB_F32, Kp, stream) == 0;
     a.src = (const float *)dense; a.R = (int)(p.nbatch * rows); a.pitch = Kp; nz = 1;
   }
@@ -1104,9 +1106,9 @@ int pb_gemm_tc_run(PbGemmProgram &p, void *const *bufs, cudaStream_t stream, int
   TcView va, vb;
   if (fp32x3) {
     if (p.dtype != PB_F32 || p.a_bf16 || p.c_bf16 || 2 * p.nbatch > 2147483647LL) return PB_TC_UNSUPPORTED;
-    va.ptr = tc_operand_x3(p, p.tc_a, bufs[p.p_a], p.off_a, true, p.M, Kp, stream, &scr_a);
+    va.ptr = tc_operand_x3(p, p.tc_a, bufs[p.p_a], p.off_a, true, p.M, Kp, fp32_mode == 3, stream, &scr_a);
     va.pitch = Kp; va.bpitch = p.M * Kp;
-    vb.ptr = va.ptr ? tc_operand_x3(p, p.tc_b, bufs[p.p_b], p.off_b, false, p.N, Kp, stream, &scr_b) : nullptr;
+    vb.ptr = va.ptr ? tc_operand_x3(p, p.tc_b, bufs[p.p_b], p.off_b, false, p.N, Kp, fp32_mode == 3, stream, &scr_b) : nullptr;
     vb.pitch = Kp; vb.bpitch = p.N * Kp;
   } else {
     Pack16Jobs jobs{};

@@ -246,7 +246,7 @@ static size_t round_size(size_t b) {
   return (b + ((size_t)2 << 20) - 1) & ~(((size_t)2 << 20) - 1);
 }
 
-static void *pool_alloc(size_t bytes) {
+static void *pool_alloc(size_t bytes, bool optional = false) {
   size_t rs = round_size(bytes);
   void *p = nullptr;
   auto it = R.free_blocks.find(rs);
@@ -261,7 +261,7 @@ static void *pool_alloc(size_t bytes) {
   else if (R.dry) { p = calloc(1, rs); }
   else if (R.capturing) {
     /* no driver allocation inside a stream capture: the caller abandons the capture */
-    R.capture_failed = true;
+    if (!optional) R.capture_failed = true;
     return nullptr;
   }
   else {
@@ -269,6 +269,7 @@ static void *pool_alloc(size_t bytes) {
     if (e != cudaSuccess) {
       /* give cached blocks back and retry once */
       cudaGetLastError();
+      if (optional) return nullptr;
       poly_b200_trim();
       e = cudaMalloc(&p, rs);
       if (e != cudaSuccess) { cudaGetLastError(); pb_set_error("cudaMalloc(%zu) failed: %s", rs, cudaGetErrorString(e)); return nullptr; }
@@ -321,6 +322,14 @@ extern "C" void poly_cuda_free(unsigned long long ptr) {
 }
 
 void *pb_scratch_alloc(size_t bytes) { return ready() ? pool_alloc(bytes) : nullptr; }
+void *pb_scratch_try(size_t bytes) { return ready() ? pool_alloc(bytes, true) : nullptr; }
+
+bool pb_captured_by_caller(void) {
+  if (!ready() || R.dry || R.capturing) return false;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(R.stream, &st) != cudaSuccess) { cudaGetLastError(); return false; }
+  return st != cudaStreamCaptureStatusNone;
+}
 void pb_scratch_free(void *p) { if (p) pool_free(p); }
 
 /* The tracked allocation containing p, or end(). */

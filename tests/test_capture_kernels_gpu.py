@@ -5,17 +5,24 @@ import ctypes
 import numpy as np
 import pytest
 
+from conftest import assert_close
 from kernel_lib import kernels  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
 
-def test_captured_chain(kernels):  # noqa: F811
-    c, P = kernels.c, ctypes.c_void_p
+def declare(c):
+    P = ctypes.c_void_p
     c.poly_b200_capture_end.restype, c.poly_b200_capture_end.argtypes = P, [ctypes.c_int]
     c.poly_b200_graph_launch.argtypes = [P, ctypes.c_ulonglong, ctypes.c_ulonglong]
     c.poly_b200_graph_destroy.restype, c.poly_b200_graph_destroy.argtypes = None, [P]
     c.poly_cuda_memset.argtypes = [ctypes.c_ulonglong, ctypes.c_ubyte, ctypes.c_size_t]
+    c.poly_b200_trim.restype, c.poly_b200_stream.restype = None, P
+    return c
+
+
+def test_captured_chain(kernels):  # noqa: F811
+    c = declare(kernels.c)
     rng = np.random.default_rng(3)
     n = 256
     x = [rng.standard_normal((n, n)).astype(np.float32) / 16 for _ in range(3)]
@@ -53,3 +60,40 @@ def test_captured_chain(kernels):  # noqa: F811
     c.poly_b200_graph_destroy(graph)
     for g, v in zip(got, want):
         assert np.array_equal(g.view(np.uint32), v.view(np.uint32))
+
+
+@pytest.mark.parametrize('whose', ['library', 'caller'])
+def test_float32_contraction_captured_before_any_call(kernels, whose):  # noqa: F811
+    """2^29 multiply-adds with nothing in the pool, in a capture of the library's or of a program that captures the
+    library's stream itself: it is recorded, and a replay reads the operands as they are then."""
+    c = declare(kernels.c)
+    rng = np.random.default_rng(4)
+    m, n, k = 1024, 1024, 516
+    a, b, d = (rng.standard_normal(s).astype(np.float32) for s in ((m, k), (k, n), (k, n)))
+    p_a, p_b, p_c = kernels.put(a), kernels.put(b), kernels.put(np.zeros((m, n), np.float32))
+
+    def call():
+        return c.poly_b200_gemm(m, n, k, p_a, k, 1, p_b, n, 1, p_c, n, None, 0, 0)
+
+    c.poly_b200_trim()
+    if whose == 'library':
+        assert c.poly_b200_capture_begin() == 0
+        rc = call()
+        graph = c.poly_b200_capture_end(0)
+        assert rc == 0 and graph, kernels.error()
+    else:
+        torch = pytest.importorskip('torch')
+        graph, status = torch.cuda.CUDAGraph(), []
+        with torch.cuda.graph(graph, stream=torch.cuda.ExternalStream(c.poly_b200_stream()), capture_error_mode='thread_local'):
+            status.append(call())
+        assert status == [0], kernels.error()
+    assert c.poly_cuda_copy_htod(p_b, d.ctypes.data, d.nbytes) == 0 and c.poly_b200_synchronize() == 0
+    if whose == 'library':
+        assert c.poly_b200_graph_launch(graph, 0, 0) == 0, kernels.error()
+    else:
+        graph.replay()
+        torch.cuda.synchronize()
+    got = kernels.get(p_c, (m, n))
+    if whose == 'library':
+        c.poly_b200_graph_destroy(graph)
+    assert_close(got, a.astype(np.float64) @ d.astype(np.float64), 1e-5, whose)
