@@ -832,7 +832,8 @@ __global__ void __launch_bounds__(256) pb200_pack16(const Pack16Jobs p) {
 /* 16-bit copy of operand A or B in a form TMA can read (v); the copy itself is added to `jobs`, or launched here
  * where the strides do not nest.  An operand whose buffer version did not change since the last
  * call (weights) is served from the program's cache; one that changes on every
- * call (activations) is converted into pool scratch that the caller frees.  0 / -1. */
+ * call (activations) is converted into pool scratch that the caller frees.  A copy recorded in a capture is
+ * not there before the replay, which may never come: it is not kept for later calls.  0 / -1. */
 static int tc_operand(PbGemmProgram &p, PbTcOperand &cache, const void *src_buf, long long off, bool is_a,
                       long long rows, cudaStream_t stream, void **scratch, Pack16Jobs &jobs, int &n_jobs, TcView *v) {
   *scratch = nullptr;
@@ -862,7 +863,7 @@ static int tc_operand(PbGemmProgram &p, PbTcOperand &cache, const void *src_buf,
     if (!cache.data) { cache.data = pb_scratch_alloc(bytes); cache.bytes = bytes; }
     if (!cache.data) return -1;
     dst = cache.data;
-    cache.form = PB_TC_FORM_16; cache.src = src_buf; cache.version = ver; cache.misses++;
+    cache.form = PB_TC_FORM_16; cache.src = src_buf; cache.version = pb_capturing() ? 0 : ver; cache.misses++;
   }
   if (plain) {
     const int esz = p.dtype == PB_F32 ? 4 : 2;
@@ -998,7 +999,7 @@ static const void *tc_operand_x3(PbGemmProgram &p, PbTcOperand &cache, const voi
     if (!cache.data) { cache.data = take(bytes); cache.bytes = bytes; }
     if (!cache.data) return nullptr;
     dst = cache.data;
-    cache.form = PB_TC_FORM_TF32; cache.src = src_buf; cache.version = ver; cache.misses++;
+    cache.form = PB_TC_FORM_TF32; cache.src = src_buf; cache.version = pb_capturing() ? 0 : ver; cache.misses++;
   }
   /* an operand whose strides nest and whose k or row axis is contiguous (an activation as the model stores it;
    * a weight; the activations a weight gradient reads transposed, whose token axes nest into one k axis) is

@@ -330,6 +330,7 @@ bool pb_captured_by_caller(void) {
   if (cudaStreamIsCapturing(R.stream, &st) != cudaSuccess) { cudaGetLastError(); return false; }
   return st != cudaStreamCaptureStatusNone;
 }
+bool pb_capturing(void) { return R.capturing || pb_captured_by_caller(); }
 void pb_scratch_free(void *p) { if (p) pool_free(p); }
 
 /* The tracked allocation containing p, or end(). */

@@ -45,6 +45,7 @@ PbAotProgram *pb_make_attn(const PbHeader &h, std::string &err);
 void *pb_scratch_alloc(size_t bytes);          /* pooled; nullptr on failure */
 void *pb_scratch_try(size_t bytes);            /* the same for callers that can do without: a failure is not reported, costs the pool
                                                   nothing and does not end a capture */
+bool  pb_capturing(void);                      /* launches are being recorded and have not run when they return */
 bool  pb_captured_by_caller(void);             /* the stream is in a capture that this library did not begin: its replays must not need
                                                   memory that the pool would hand out again, nor copies made before it */
 void  pb_scratch_free(void *p);

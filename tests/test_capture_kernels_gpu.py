@@ -97,3 +97,28 @@ def test_float32_contraction_captured_before_any_call(kernels, whose):  # noqa: 
     if whose == 'library':
         c.poly_b200_graph_destroy(graph)
     assert_close(got, a.astype(np.float64) @ d.astype(np.float64), 1e-5, whose)
+
+
+@pytest.mark.parametrize('policy,m,n,k', [(1, 136, 64, 64), (0, 1096, 1024, 512), (0, 1096, 1024, 1024)], ids=str)
+@pytest.mark.parametrize('discard', [0, 1])
+def test_call_after_a_capture_that_never_ran(kernels, policy, m, n, k, discard):  # noqa: F811
+    """Operand copies that a capture recorded and nothing replayed are not taken for the operands'."""
+    c = declare(kernels.c)
+    c.poly_b200_set_gemm_policy(policy)
+    m += 64 * discard                         # a program of its own each time
+    rng = np.random.default_rng(5)
+    # small whole numbers: every route gives the same result
+    x = [rng.integers(-4, 5, s).astype(np.float32) for s in ((m, k), (k, n), (m, k), (k, n))]
+    p_x, p_c = [kernels.put(v) for v in x], kernels.put(np.zeros((m, n), np.float32))
+
+    def call(i):
+        assert c.poly_b200_gemm(m, n, k, p_x[i], k, 1, p_x[i + 1], n, 1, p_c, n, None, 0, 0) == 0, kernels.error()
+
+    call(0)                                   # the program and its memory exist
+    assert c.poly_b200_capture_begin() == 0
+    call(2)
+    graph = c.poly_b200_capture_end(discard)
+    assert bool(graph) != bool(discard)
+    c.poly_b200_graph_destroy(graph)
+    call(2)
+    assert np.array_equal(kernels.get(p_c, (m, n)), x[2] @ x[3])
