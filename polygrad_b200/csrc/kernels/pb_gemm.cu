@@ -494,7 +494,7 @@ template <bool AK, bool BKm>
 static int small_launch(const SgemmArgs &g, dim3 grid, int n_split, bool wide_a, bool wide_b, cudaStream_t stream) {
   static bool configured = false;
   cudaError_t e = cudaSuccess;
-  if (!configured) { e = cudaFuncSetAttribute(pb200_sgemm_small<AK, BKm>, cudaFuncAttributeMaxDynamicSharedMemorySize, S_SMEM); configured = e == cudaSuccess; }
+  if (!configured) { e = cudaFuncSetAttribute(pb200_sgemm_small<AK, BKm>, cudaFuncAttributeMaxDynamicSharedMemorySize, S_SMEM); configured = e == cudaSuccess; if (!configured) cudaGetLastError(); }
   if (e == cudaSuccess) e = pb_launch_chained(pb200_sgemm_small<AK, BKm>, dim3(grid.x * (unsigned)n_split, grid.y, grid.z), 256, S_SMEM, stream, (unsigned)n_split, g, n_split, wide_a, wide_b);
   if (e != cudaSuccess) { pb_set_error("sgemm launch: %s", cudaGetErrorString(e)); return -1; }
   return 0;

@@ -31,7 +31,9 @@ static inline cudaError_t pb_launch_chained(F *kernel, dim3 grid, unsigned threa
   attr[1].id = cudaLaunchAttributeClusterDimension;
   attr[1].val.clusterDim.x = cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr; cfg.numAttrs = cluster > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+  if (e != cudaSuccess) cudaGetLastError();        /* returned here: not the next launch's error as well */
+  return e;
 }
 #ifdef __CUDACC__
 __device__ __forceinline__ void pb_grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
