@@ -979,25 +979,25 @@ __global__ void __launch_bounds__(256) pb200_split_tf32(const SplitArgs a) {
 }
 
 /* The two parts of A or B, [2][nbatch][rows][Kp] float32; cached like the bf16 copies.  optional: the caller has another
- * way when the pool has no memory for them. */
-static const void *tc_operand_x3(PbGemmProgram &p, PbTcOperand &cache, const void *src_buf, long long off, bool is_a,
-                                 long long rows, long long Kp, bool optional, cudaStream_t stream, void **scratch) {
+ * way when the pool has no memory for them.  0, -1 or PB_TC_NO_SCRATCH. */
+static int tc_operand_x3(PbGemmProgram &p, PbTcOperand &cache, const void *src_buf, long long off, bool is_a,
+                         long long rows, long long Kp, bool optional, cudaStream_t stream, void **scratch, const void **parts) {
   void *(*const take)(size_t) = optional ? pb_scratch_try : pb_scratch_alloc;
   *scratch = nullptr;
   const size_t bytes = (size_t)(p.nbatch * rows * 2 * Kp) * 4;
   const uint64_t ver = pb_buffer_version(src_buf);
-  if (cache.data && cache.form == PB_TC_FORM_TF32 && cache.src == src_buf && cache.version == ver && cache.bytes == bytes && ver != 0) return cache.data;
+  if (cache.data && cache.form == PB_TC_FORM_TF32 && cache.src == src_buf && cache.version == ver && cache.bytes == bytes && ver != 0) { *parts = cache.data; return 0; }
   const bool transient = cache.misses >= 2 || ver == 0;
   void *dst;
   if (transient) {
     if (cache.data) { pb_scratch_free(cache.data); cache.data = nullptr; cache.bytes = 0; }
     dst = take(bytes);
-    if (!dst) return nullptr;
+    if (!dst) return PB_TC_NO_SCRATCH;
     *scratch = dst;
   } else {
     if (cache.data && cache.bytes != bytes) { pb_scratch_free(cache.data); cache.data = nullptr; }
     if (!cache.data) { cache.data = take(bytes); cache.bytes = bytes; }
-    if (!cache.data) return nullptr;
+    if (!cache.data) return PB_TC_NO_SCRATCH;
     dst = cache.data;
     cache.form = PB_TC_FORM_TF32; cache.src = src_buf; cache.version = pb_capturing() ? 0 : ver; cache.misses++;
   }
@@ -1014,7 +1014,7 @@ static const void *tc_operand_x3(PbGemmProgram &p, PbTcOperand &cache, const voi
   long long nz = 1;
   for (auto &b : p.b_ax) { if (sel(b) < 0) in_place = false; nz *= b.ext; }
   void *dense = nullptr;
-  bool ok = true;
+  int rc = 0;
   SplitArgs a{};
   a.dst = (float *)dst; a.plane = p.nbatch * rows * Kp; a.K = (int)p.K; a.Kp = (int)Kp;
   if (in_place) {
@@ -1022,27 +1022,29 @@ static const void *tc_operand_x3(PbGemmProgram &p, PbTcOperand &cache, const voi
     a.pitch = kfast ? (rows > 1 ? srow : 0) : sk;
     for (auto &b : p.b_ax) { a.ext[a.naxes] = (int)b.ext; a.sstride[a.naxes++] = sel(b); }
   } else {
-    if (p.nbatch * rows > 2147483647LL - 64) ok = false;
-    dense = ok ? take((size_t)(p.nbatch * rows * Kp) * 4) : nullptr;
-    ok = dense != nullptr && p.pack_into(dense, src_buf, off, is_a, PB_F32, PB_F32, Kp, stream) == 0;
+    if (p.nbatch * rows > 2147483647LL - 64) { pb_set_error("gemm: operand too large to split"); rc = -1; }
+    dense = rc == 0 ? take((size_t)(p.nbatch * rows * Kp) * 4) : nullptr;
+    if (rc == 0) rc = !dense ? PB_TC_NO_SCRATCH : p.pack_into(dense, src_buf, off, is_a, PB_F32, PB_F32, Kp, stream);
     a.src = (const float *)dense; a.R = (int)(p.nbatch * rows); a.pitch = Kp; nz = 1;
   }
   a.vec = (reinterpret_cast<uintptr_t>(a.src) & 15) == 0 && a.pitch % 4 == 0;
   for (int i = 0; i < a.naxes; i++) if (a.sstride[i] % 4) a.vec = 0;
   a.tr = (a.R + 63) / 64; a.tk = ((int)Kp + 63) / 64;
   const long long blocks = (long long)a.tr * a.tk * nz;
-  if (blocks > 2147483647LL) { pb_set_error("gemm: operand too large to split"); ok = false; }
-  if (ok) {
-    ok = pb_launch_chained(in_place && !kfast ? pb200_split_tf32<false> : pb200_split_tf32<true>, dim3((unsigned)blocks), 256, 0, stream, 1, a) == cudaSuccess;
+  if (rc == 0 && blocks > 2147483647LL) { pb_set_error("gemm: operand too large to split"); rc = -1; }
+  if (rc == 0) {
+    const cudaError_t err = pb_launch_chained(in_place && !kfast ? pb200_split_tf32<false> : pb200_split_tf32<true>, dim3((unsigned)blocks), 256, 0, stream, 1, a);
+    if (err != cudaSuccess) { pb_set_error("gemm: operand split launch: %s", cudaGetErrorString(err)); rc = -1; }
     p.launches++;
   }
   pb_scratch_free(dense);           /* stream-ordered pool: reusable by later work on this stream */
-  if (!ok) {
+  if (rc != 0) {
     if (*scratch) { pb_scratch_free(*scratch); *scratch = nullptr; }
     else cache.version = 0;
-    return nullptr;
+    return rc;
   }
-  return dst;
+  *parts = dst;
+  return 0;
 }
 
 static bool tc_in_place(const PbGemmProgram &p, const void *buf, long long off, bool is_a, TcView *v) {
@@ -1107,9 +1109,10 @@ int pb_gemm_tc_run(PbGemmProgram &p, void *const *bufs, cudaStream_t stream, int
   TcView va, vb;
   if (fp32x3) {
     if (p.dtype != PB_F32 || p.a_bf16 || p.c_bf16 || 2 * p.nbatch > 2147483647LL) return PB_TC_UNSUPPORTED;
-    va.ptr = tc_operand_x3(p, p.tc_a, bufs[p.p_a], p.off_a, true, p.M, Kp, fp32_mode == 3, stream, &scr_a);
+    int rc = tc_operand_x3(p, p.tc_a, bufs[p.p_a], p.off_a, true, p.M, Kp, fp32_mode == 3, stream, &scr_a, &va.ptr);
+    if (rc == 0) rc = tc_operand_x3(p, p.tc_b, bufs[p.p_b], p.off_b, false, p.N, Kp, fp32_mode == 3, stream, &scr_b, &vb.ptr);
+    if (rc != 0) { pb_scratch_free(scr_a); return rc; }
     va.pitch = Kp; va.bpitch = p.M * Kp;
-    vb.ptr = va.ptr ? tc_operand_x3(p, p.tc_b, bufs[p.p_b], p.off_b, false, p.N, Kp, fp32_mode == 3, stream, &scr_b) : nullptr;
     vb.pitch = Kp; vb.bpitch = p.N * Kp;
   } else {
     Pack16Jobs jobs{};
@@ -1147,7 +1150,7 @@ int pb_gemm_tc_run(PbGemmProgram &p, void *const *bufs, cudaStream_t stream, int
       }
     }
   }
-  if (!va.ptr || !vb.ptr) { pb_scratch_free(scr_a); pb_scratch_free(scr_b); return fp32x3 ? PB_TC_NO_SCRATCH : -1; }
+  if (!va.ptr || !vb.ptr) { pb_scratch_free(scr_a); pb_scratch_free(scr_b); return -1; }
 
   TcArgs g{};
   long long rowsA = p.M, rowsB = p.N;
