@@ -907,8 +907,8 @@ __device__ __forceinline__ void split_one(float a, float &hi, float &lo) {
   if (!(fabsf(a) <= 3.4028235e38f)) {
     /* an infinity or a NaN is the lo part beside a hi part of its sign: it then meets the other operand's hi
      * part once (inf * b keeps b's sign, inf * 0 is NaN) and never a lo part, which has either sign; two
-     * infinities meet as 1 * inf + inf * 1 */
-    hi = copysignf(1.0f, a); lo = a;
+     * infinities meet as 1 * inf + inf * 1.  (A NaN may differ from an infinity only in bits that tf32 leaves out.) */
+    hi = copysignf(1.0f, a); lo = a != a ? __int_as_float(0x7fc00000) : a;
     return;
   }
   hi = tf32_rna(a);

@@ -214,3 +214,16 @@ def test_f32_default_route_errs_no_more_than_sums_in_k_order(kernels, m, n, k, v
         acc = (acc + np.outer(x[:, i], y[:, i])).astype(np.float32)
     err = [np.sqrt(np.mean((v - x @ y.T) ** 2)) for v in (kernels.get(c, (m, n))[np.ix_(rows, cols)], acc)]
     assert err[0] <= 1.1 * err[1]
+
+
+def test_f32_nan_of_any_payload(kernels):  # noqa: F811
+    """A NaN that differs from an infinity only in bits that tf32 does not hold stays a NaN (2^29 multiply-adds, default route)."""
+    m, n, k = 1024, 1024, 512
+    rng = np.random.default_rng(6)
+    a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((k, n)).astype(np.float32)
+    a.view(np.uint32)[3, 5], a.view(np.uint32)[700, 500], b.view(np.uint32)[9, 77] = 0x7f800001, 0xff801fff, 0x7f801000
+    c = kernels.put(np.zeros((m, n), np.float32))
+    assert kernels.c.poly_b200_gemm(m, n, k, kernels.put(a), k, 1, kernels.put(b), n, 1, c, n, None, 0, 0) == 0, kernels.error()
+    want = np.zeros((m, n), bool)
+    want[[3, 700], :] = want[:, 77] = True
+    assert np.array_equal(np.isnan(kernels.get(c, (m, n))), want)
