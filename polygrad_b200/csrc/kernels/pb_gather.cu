@@ -47,6 +47,7 @@ template <bool FLAT>
 __device__ __forceinline__ void gather_token(const GatherArgs &a, long long tok, long long *o_out, long long *o_ids) {
   if (FLAT) { *o_out = a.out_off + tok * a.tok_out[0]; *o_ids = a.ids_off + tok * a.tok_ids[0]; return; }
   *o_out = a.out_off; *o_ids = a.ids_off;
+  if (a.ntok == 1) { *o_out += tok * a.tok_out[0]; *o_ids += tok * a.tok_ids[0]; return; }
   for (int i = 0; i < a.ntok; i++) {
     const long long x = tok % a.tok_ext[i]; tok /= a.tok_ext[i];
     *o_out += x * a.tok_out[i]; *o_ids += x * a.tok_ids[i];
@@ -126,50 +127,105 @@ __global__ void __launch_bounds__(GATHER_THREADS) pb200_gather_rows(const Gather
   if (!ok) pb200_gather_state[0] = 1;
 }
 
-/* Any `arange`: every block searches all of it for its tokens. */
+/* Any `arange`: a block searches all of it for up to four tokens at a time, eight values per thread in flight and eight being
+ * compared; its warps then share the rows.  Bound by the compares and L2 round trips.  8192 tokens of a 50257 x 768 table, numbering permuted, the
+ * first kernel's 11 us included: 196 us with one token and value at a time, 86 like this (172 where a block per token
+ * searched at once and no rows had been copied before); 16 tokens 24 and 18 (25). */
+#define GATHER_SEARCH_TOKENS 4
+#define GATHER_SEARCH_DEEP 8
+template <bool FLAT>
 __global__ void __launch_bounds__(GATHER_THREADS) pb200_gather_search(const GatherArgs a) {
-  __shared__ int s_count;
-  __shared__ long long s_match[GATHER_MAX_MATCH];
+  __shared__ int s_count[GATHER_SEARCH_TOKENS];
+  __shared__ long long s_out[GATHER_SEARCH_TOKENS], s_match[GATHER_SEARCH_TOKENS][GATHER_MAX_MATCH];
+  __shared__ float s_id[GATHER_SEARCH_TOKENS];
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (*(volatile int *)pb200_gather_state == 0) return;
-  for (long long tok = blockIdx.x; tok < a.n_tokens; tok += gridDim.x) {
-    long long o_out, o_ids;
-    gather_token<false>(a, tok, &o_out, &o_ids);
-    if (threadIdx.x == 0) s_count = 0;
-    __syncthreads();
-    const float id = a.ids[o_ids];
-    for (long long v = threadIdx.x; v < a.vocab; v += GATHER_THREADS) {
-      if (a.arange[v] == id) {
-        const int slot = atomicAdd(&s_count, 1);
-        if (slot < GATHER_MAX_MATCH) s_match[slot] = v;
+  const int per = (int)min((long long)GATHER_SEARCH_TOKENS, (a.n_tokens + gridDim.x - 1) / gridDim.x);
+  for (long long tok0 = (long long)blockIdx.x * per; tok0 < a.n_tokens; tok0 += (long long)gridDim.x * per) {
+    const int n = (int)min((long long)per, a.n_tokens - tok0);
+    if (threadIdx.x < GATHER_SEARCH_TOKENS) {
+      s_count[threadIdx.x] = 0;
+      s_id[threadIdx.x] = __int_as_float(0x7fc00000);        /* matches nothing */
+      if ((int)threadIdx.x < n) {
+        long long o_ids;
+        gather_token<false>(a, tok0 + threadIdx.x, &s_out[threadIdx.x], &o_ids);
+        s_id[threadIdx.x] = a.ids[o_ids];
       }
     }
     __syncthreads();
-    const int count = s_count;
-    if (count > 1 && count <= GATHER_MAX_MATCH && threadIdx.x == 0) {
+    float id[GATHER_SEARCH_TOKENS];
+#pragma unroll
+    for (int i = 0; i < GATHER_SEARCH_TOKENS; i++) id[i] = s_id[i];
+    float x[GATHER_SEARCH_DEEP], next[GATHER_SEARCH_DEEP];
+    auto fetch = [&](long long v0) {                         /* values v0 + threadIdx.x + j * 256 */
+      const float *p = a.arange + v0 + threadIdx.x;
+      const int left = (int)min((long long)(GATHER_THREADS * GATHER_SEARCH_DEEP), a.vocab - v0) - (int)threadIdx.x;
+#pragma unroll
+      for (int j = 0; j < GATHER_SEARCH_DEEP; j++) next[j] = j * GATHER_THREADS < left ? __ldg(p + j * GATHER_THREADS) : __int_as_float(0x7fc00000);
+    };
+    fetch(0);
+    for (long long v0 = 0; v0 < a.vocab; v0 += GATHER_THREADS * GATHER_SEARCH_DEEP) {
+#pragma unroll
+      for (int j = 0; j < GATHER_SEARCH_DEEP; j++) x[j] = next[j];
+      if (v0 + GATHER_THREADS * GATHER_SEARCH_DEEP < a.vocab) fetch(v0 + GATHER_THREADS * GATHER_SEARCH_DEEP);
+      bool any = false;
+#pragma unroll
+      for (int j = 0; j < GATHER_SEARCH_DEEP; j++) any |= x[j] == id[0] || x[j] == id[1] || x[j] == id[2] || x[j] == id[3];
+      if (any) {
+#pragma unroll
+        for (int j = 0; j < GATHER_SEARCH_DEEP; j++)
+#pragma unroll 1
+          for (int i = 0; i < n; i++)
+            if (x[j] == s_id[i]) {
+              const int slot = atomicAdd(&s_count[i], 1);
+              if (slot < GATHER_MAX_MATCH) s_match[i][slot] = v0 + threadIdx.x + j * GATHER_THREADS;
+            }
+      }
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < n && s_count[threadIdx.x] <= GATHER_MAX_MATCH) {
       /* ascending v: the order the reference adds in */
-      for (int i = 1; i < count; i++) {
-        long long x = s_match[i]; int j = i - 1;
-        while (j >= 0 && s_match[j] > x) { s_match[j + 1] = s_match[j]; j--; }
-        s_match[j + 1] = x;
+      long long *m = s_match[threadIdx.x];
+      for (int i = 1; i < s_count[threadIdx.x]; i++) {
+        long long x = m[i]; int j = i - 1;
+        while (j >= 0 && m[j] > x) { m[j + 1] = m[j]; j--; }
+        m[j + 1] = x;
       }
     }
     __syncthreads();
-    for (long long f = threadIdx.x; f < a.n_feat; f += GATHER_THREADS) {
-      long long fr = f, o = o_out, t = a.table_off;
-      for (int i = 0; i < a.nfeat; i++) {
-        const long long x = fr % a.feat_ext[i]; fr /= a.feat_ext[i];
-        o += x * a.feat_out[i]; t += x * a.feat_tab[i];
-      }
-      float acc = 0.0f;
-      if (count <= GATHER_MAX_MATCH) {
-        for (int i = 0; i < count; i++) acc = acc + a.table[t + s_match[i] * a.table_vstride];
+    const int warp = threadIdx.x >> 5, parts = GATHER_THREADS / 32 / n, k = warp % n, part = warp / n;      /* warps share the rows */
+    const int count = s_count[k];
+    if (part < parts) {
+      const long long step = parts * 32, f0 = part * 32 + (threadIdx.x & 31);
+      if (FLAT && count <= 1) {
+        const float *t = a.table + a.table_off + (count ? s_match[k][0] : 0) * a.table_vstride;
+        float *o = a.out + s_out[k];
+        for (long long f = f0; f < a.n_feat; f += step * 8) {
+          float x[8];
+#pragma unroll
+          for (int i = 0; i < 8; i++) x[i] = count && f + i * step < a.n_feat ? __ldg(t + f + i * step) : 0.0f;
+#pragma unroll
+          for (int i = 0; i < 8; i++) if (f + i * step < a.n_feat) o[f + i * step] = 0.0f + x[i];
+        }
       } else {
-        /* pathological arange with many duplicates: plain ordered scan */
-        for (long long v = 0; v < a.vocab; v++)
-          if (a.arange[v] == id) acc = acc + a.table[t + v * a.table_vstride];
+        for (long long f = f0; f < a.n_feat; f += step) {
+          long long fr = f, o = s_out[k], t = a.table_off;
+          if (FLAT) { o += f; t += f; }
+          else for (int i = 0; i < a.nfeat; i++) {
+            const long long x = fr % a.feat_ext[i]; fr /= a.feat_ext[i];
+            o += x * a.feat_out[i]; t += x * a.feat_tab[i];
+          }
+          float acc = 0.0f;
+          if (count <= GATHER_MAX_MATCH) {
+            for (int i = 0; i < count; i++) acc = acc + a.table[t + s_match[k][i] * a.table_vstride];
+          } else {
+            /* pathological arange with many duplicates: plain ordered scan */
+            for (long long v = 0; v < a.vocab; v++)
+              if (a.arange[v] == s_id[k]) acc = acc + a.table[t + v * a.table_vstride];
+          }
+          a.out[o] = acc;
+        }
       }
-      a.out[o] = acc;
     }
     __syncthreads();
   }
@@ -221,7 +277,7 @@ struct GatherProgram : PbAotProgram {
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, pb200_gather_search, g);
+    cudaLaunchKernelEx(&cfg, flat ? pb200_gather_search<true> : pb200_gather_search<false>, g);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { pb_set_error("gather launch: %s", cudaGetErrorString(e)); return -1; }
     return 0;

@@ -25,7 +25,7 @@ def numbering(kind, vocab, rng):
 
 
 SIZES = [(1, 4, 1, 1), (5, 7, 1, 3), (64, 64, 2, 33), (65, 96, 1, 4097), (130, 768, 3, 50), (1000, 1604, 1, 17), (257, 1028, 2, 100),
-         (40, 128, 1, 9000)]
+         (40, 128, 1, 9000), (33, 20, 1, 700), (70, 36, 1, 1500)]
 
 
 @pytest.mark.parametrize('kind', ['plain', 'shifted', 'permuted', 'repeated'])
