@@ -323,9 +323,9 @@ PbAotProgram *pb_make_gather(const PbHeader &h, std::string &err) {
  * the result so far in later chunks) -- the order and the value of the reference's accumulation, in which the
  * non-matching tokens add +0 -- with SCATTER_DEEP rows' loads in flight.
  *
- * A token finds its row by subtraction where the block's part of `arange` is consecutive integers, by
- * comparing with every row where its values are merely distinct (NaNs match nothing); where values repeat, one
- * token matches several rows and the rows are taken one at a time.  A warp's list holds every token of its part
+ * A token finds its row by subtraction where the block's part of `arange` is consecutive integers, otherwise by
+ * comparing with every row (NaNs match nothing); where values repeat, the tokens go to the last row of their value, whose
+ * sum the others copy.  A warp's list holds every token of its part
  * of a chunk, so it cannot overflow.
  *
  * HBM traffic: the output written once, the ids read once per block (from L2), the matching source rows.  8192
@@ -360,7 +360,8 @@ __global__ void __launch_bounds__(SCATTER_THREADS, 4) pb200_scatter_rows(const S
   __shared__ __align__(16) int s_off[SCATTER_ROWS * SCATTER_WARPS];   /* matches of (row, warp): their number, then where they go in s_tok */
   __shared__ int s_begin[SCATTER_ROWS + 1];                       /* where those of the row begin */
   __shared__ unsigned char s_rows[SCATTER_ROWS];                  /* rows with matches */
-  __shared__ int s_matched;
+  __shared__ int s_matched, s_distinct;
+  __shared__ unsigned char s_some[SCATTER_ROWS];                  /* rows that had matches in any chunk */
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long v0 = (long long)blockIdx.x * a.rows_per_block;
   const int rows = (int)min((long long)a.rows_per_block, a.vocab - v0);
@@ -382,182 +383,192 @@ __global__ void __launch_bounds__(SCATTER_THREADS, 4) pb200_scatter_rows(const S
     if (MODE == 2) for (int f = lane * 4; f < nf; f += 128) *reinterpret_cast<float4 *>(orow + f_begin + f) = make_float4(0.f, 0.f, 0.f, 0.f);
     else for (int f = lane; f < nf; f += 32) { feature(f, &oo, &so); orow[oo] = 0.0f; }
   }
-  if (threadIdx.x < SCATTER_ROWS) s_ar[threadIdx.x] = (int)threadIdx.x < rows ? a.arange[v0 + threadIdx.x] : __int_as_float(0x7fc00000);
+  if (threadIdx.x < SCATTER_ROWS) {
+    s_ar[threadIdx.x] = (int)threadIdx.x < rows ? a.arange[v0 + threadIdx.x] : __int_as_float(0x7fc00000);
+    s_some[threadIdx.x] = 0;
+  }
+  if (threadIdx.x == 0) s_distinct = 1;
   __syncthreads();
   const float ar0 = s_ar[0];
-  bool consecutive = truncf(ar0) == ar0 && fabsf(ar0) < 8388608.0f, distinct = true;      /* differences of such values are exact */
+  bool consecutive = truncf(ar0) == ar0 && fabsf(ar0) < 8388608.0f;        /* differences of such values are exact */
   if ((int)threadIdx.x < rows) consecutive &= s_ar[threadIdx.x] == ar0 + (float)threadIdx.x;
   consecutive = __syncthreads_and(consecutive ? 1 : 0) != 0;
-  if (!consecutive) {
-    if ((int)threadIdx.x < rows) for (int r = 0; r < (int)threadIdx.x; r++) distinct &= s_ar[r] != s_ar[threadIdx.x];
-    distinct = __syncthreads_and(distinct ? 1 : 0) != 0;
-  }
-  const int group = distinct ? rows : 1;                                   /* rows taken together */
-
-  for (int r0 = 0; r0 < rows; r0 += group) {
-    auto row_of = [&](float x) {
-      if (consecutive) { const float dlt = x - ar0; return dlt >= 0.0f && dlt < (float)rows && ar0 + dlt == x && truncf(dlt) == dlt ? (int)dlt : -1; }
-      if (!distinct) return x == s_ar[r0] ? 0 : -1;
-      int row = -1;
-      for (int r = 0; r < rows; r++) if (x == s_ar[r]) row = r;
-      return row;
-    };
-    for (long long c0 = 0; c0 < a.n_tokens; c0 += SCATTER_CHUNK) {
-      /* matches of this warp's tokens: four consecutive tokens per lane and step, all steps' loads in flight */
-      const long long w0 = c0 + warp * PER_WARP;
-      const int nw = (int)max(0LL, min((long long)PER_WARP, a.n_tokens - w0));
-      float id[PER_WARP / 128][4];
+  if (!consecutive && (int)threadIdx.x < rows)
+    for (int r = 0; r < (int)threadIdx.x; r++) if (s_ar[r] == s_ar[threadIdx.x]) s_distinct = 0;
+  /* the last row of the token's value */
+  auto row_of = [&](float x) {
+    if (consecutive) { const float dlt = x - ar0; return dlt >= 0.0f && dlt < (float)rows && ar0 + dlt == x && truncf(dlt) == dlt ? (int)dlt : -1; }
+    int row = -1;
+    for (int r = 0; r < rows; r++) if (x == s_ar[r]) row = r;
+    return row;
+  };
+  for (long long c0 = 0; c0 < a.n_tokens; c0 += SCATTER_CHUNK) {
+    /* matches of this warp's tokens: four consecutive tokens per lane and step, all steps' loads in flight */
+    const long long w0 = c0 + warp * PER_WARP;
+    const int nw = (int)max(0LL, min((long long)PER_WARP, a.n_tokens - w0));
+    float id[PER_WARP / 128][4];
 #pragma unroll
-      for (int s = 0; s < PER_WARP / 128; s++) {
-        const int t = s * 128 + lane * 4;
-        if (a.ids_vec && t + 3 < nw) {
-          const float4 x = __ldg(reinterpret_cast<const float4 *>(a.ids + a.ids_off + w0 + t));
-          id[s][0] = x.x; id[s][1] = x.y; id[s][2] = x.z; id[s][3] = x.w;
-        } else {
+    for (int s = 0; s < PER_WARP / 128; s++) {
+      const int t = s * 128 + lane * 4;
+      if (a.ids_vec && t + 3 < nw) {
+        const float4 x = __ldg(reinterpret_cast<const float4 *>(a.ids + a.ids_off + w0 + t));
+        id[s][0] = x.x; id[s][1] = x.y; id[s][2] = x.z; id[s][3] = x.w;
+      } else {
 #pragma unroll
-          for (int i = 0; i < 4; i++) {
-            id[s][i] = __int_as_float(0x7fc00000);                         /* matches nothing */
-            if (t + i < nw) {
-              long long rem = w0 + t + i, o = a.ids_off;
-              if (MODE) o += rem * a.tok_ids[0];
-              else for (int d = 0; d < a.ntok; d++) { const long long x = rem % a.tok_ext[d]; rem /= a.tok_ext[d]; o += x * a.tok_ids[d]; }
-              id[s][i] = a.ids[o];
-            }
+        for (int i = 0; i < 4; i++) {
+          id[s][i] = __int_as_float(0x7fc00000);                         /* matches nothing */
+          if (t + i < nw) {
+            long long rem = w0 + t + i, o = a.ids_off;
+            if (MODE) o += rem * a.tok_ids[0];
+            else for (int d = 0; d < a.ntok; d++) { const long long x = rem % a.tok_ext[d]; rem /= a.tok_ext[d]; o += x * a.tok_ids[d]; }
+            id[s][i] = a.ids[o];
           }
         }
       }
-      for (int i = threadIdx.x; i < SCATTER_ROWS * SCATTER_WARPS / 4; i += SCATTER_THREADS) reinterpret_cast<int4 *>(s_off)[i] = make_int4(0, 0, 0, 0);
-      __syncthreads();
-      int n = 0;                                                           /* entries of this warp's list */
-#pragma unroll
-      for (int s = 0; s < PER_WARP / 128; s++) {
-        int row[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) row[i] = row_of(id[s][i]);
-        const int mine = (row[0] >= 0) + (row[1] >= 0) + (row[2] >= 0) + (row[3] >= 0);
-        if (__any_sync(0xffffffffu, mine)) {
-          int at = mine;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, at, o); if (lane >= o) at += y; }
-          const int total = __shfl_sync(0xffffffffu, at, 31);
-          at += n - mine;
-#pragma unroll
-          for (int i = 0; i < 4; i++)
-            if (row[i] >= 0) {
-              s_list[warp][at++] = ((unsigned)row[i] << 16) | (unsigned)(warp * PER_WARP + s * 128 + lane * 4 + i);
-              atomicAdd(&s_off[row[i] * SCATTER_WARPS + warp], 1);
-            }
-          n += total;
-        }
-      }
-      __syncthreads();
-      /* counts -> positions, by row and, within a row, by warp (which is by token); a lane per row */
-      if (warp == 0) {
-        int base = 0, found = 0;
-#pragma unroll 1
-        for (int rb = 0; rb < SCATTER_ROWS && rb < rows; rb += 32) {
-          int4 *cp = reinterpret_cast<int4 *>(s_off + (rb + lane) * SCATTER_WARPS);
-          const int4 c = cp[0], d = cp[1];
-          const int sum = c.x + c.y + c.z + c.w + d.x + d.y + d.z + d.w;
-          int at = sum;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, at, o); if (lane >= o) at += y; }
-          const int total = __shfl_sync(0xffffffffu, at, 31);
-          at += base - sum;
-          s_begin[rb + lane] = at;
-          const unsigned some = __ballot_sync(0xffffffffu, sum > 0);
-          if (sum > 0) s_rows[found + __popc(some & ((1u << lane) - 1u))] = (unsigned char)(rb + lane);
-          int4 p, q;
-          p.x = at; p.y = p.x + c.x; p.z = p.y + c.y; p.w = p.z + c.z; q.x = p.w + c.w; q.y = q.x + d.x; q.z = q.y + d.y; q.w = q.z + d.z;
-          cp[0] = p; cp[1] = q;
-          base += total; found += __popc(some);
-        }
-        if (lane == 0) { s_begin[min(SCATTER_ROWS, (rows + 31) / 32 * 32)] = base; s_matched = found; }
-      }
-      __syncthreads();
-      /* every warp places its list; s_off[row, warp] moves on with it */
-      for (int i0 = 0; i0 < n; i0 += 32) {
-        const bool have = i0 + lane < n;
-        const unsigned e = have ? s_list[warp][i0 + lane] : 0xffffffffu;
-        const unsigned peers = __match_any_sync(0xffffffffu, e >> 16);
-        const int before = __popc(peers & ((1u << lane) - 1u));
-        int *slot = &s_off[(e >> 16) * SCATTER_WARPS + warp];
-        int at = 0;
-        if (have) { at = *slot; s_tok[at + before] = (unsigned short)(e & 0xffffu); }
-        __syncwarp();
-        if (have && before == 0) *slot = at + __popc(peers);
-        __syncwarp();
-      }
-      __syncthreads();
-      auto token_row = [&](int m) {
-        long long rem = c0 + s_tok[m];
-        if (MODE) return src + rem * a.tok_src[0];
-        const float *p = src;
-        for (int d = 0; d < a.ntok; d++) { const long long x = rem % a.tok_ext[d]; rem /= a.tok_ext[d]; p += x * a.tok_src[d]; }
-        return p;
-      };
-      const int matched = s_matched;
-      /* the source rows of the commonest words are requested from memory beforehand: their sum is one serial chain */
-      if (MODE) {
-        const unsigned lines = ((unsigned)nf + 31) / 32;
-        for (int k = 0; k < matched; k++) {
-          const int m0 = s_begin[s_rows[k]], m1 = s_begin[s_rows[k] + 1];
-          if (m1 - m0 <= SCATTER_DEEP) continue;
-          for (unsigned i = threadIdx.x; i < (unsigned)(m1 - m0) * lines; i += SCATTER_THREADS) {
-            const unsigned m = i / lines;
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(token_row(m0 + (int)m) + f_begin + (i - m * lines) * 32));
-          }
-        }
-      }
-      for (unsigned item = warp; item < (unsigned)(matched * segs); item += SCATTER_WARPS) {
-        const unsigned k = item / (unsigned)segs;
-        const int r = s_rows[k], f = (int)(item - k * segs) * 128 + (MODE == 2 ? lane * 4 : lane);
-        const int m0 = s_begin[r], m1 = s_begin[r + 1];
-        float *orow = out + (r0 + r) * a.out_vstride;
-        if (MODE == 2) {
-          if (f >= nf) continue;
-          float4 *op = reinterpret_cast<float4 *>(orow + f_begin + f);
-          float4 acc = c0 == 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : *op;
-          for (int m = m0; m < m1; m += SCATTER_DEEP) {
-            float4 x[SCATTER_DEEP];
-#pragma unroll
-            for (int i = 0; i < SCATTER_DEEP; i++) if (m + i < m1) x[i] = __ldg(reinterpret_cast<const float4 *>(token_row(m + i) + f_begin + f));
-#pragma unroll
-            for (int i = 0; i < SCATTER_DEEP; i++) if (m + i < m1) { acc.x += x[i].x; acc.y += x[i].y; acc.z += x[i].z; acc.w += x[i].w; }
-          }
-          *op = acc;
-        } else {
-          /* four features 32 apart per lane */
-          long long oo[4], so[4];
-          float acc[4];
-#pragma unroll
-          for (int j = 0; j < 4; j++) {
-            feature(f + j * 32, &oo[j], &so[j]);
-            acc[j] = (c0 == 0 || f + j * 32 >= nf) ? 0.0f : orow[oo[j]];
-          }
-          constexpr int DEEP = MODE ? 4 : 1;
-          for (int m = m0; m < m1; m += DEEP) {
-            float x[DEEP][4];
-#pragma unroll
-            for (int i = 0; i < DEEP; i++)
-              if (m + i < m1) {
-                const float *p = token_row(m + i);
-#pragma unroll
-                for (int j = 0; j < 4; j++) if (f + j * 32 < nf) x[i][j] = __ldg(p + so[j]);
-              }
-#pragma unroll
-            for (int i = 0; i < DEEP; i++)
-              if (m + i < m1) {
-#pragma unroll
-                for (int j = 0; j < 4; j++) if (f + j * 32 < nf) acc[j] += x[i][j];
-              }
-          }
-#pragma unroll
-          for (int j = 0; j < 4; j++) if (f + j * 32 < nf) orow[oo[j]] = acc[j];
-        }
-      }
-      __syncthreads();
     }
+    for (int i = threadIdx.x; i < SCATTER_ROWS * SCATTER_WARPS / 4; i += SCATTER_THREADS) reinterpret_cast<int4 *>(s_off)[i] = make_int4(0, 0, 0, 0);
+    __syncthreads();
+    int n = 0;                                                           /* entries of this warp's list */
+#pragma unroll
+    for (int s = 0; s < PER_WARP / 128; s++) {
+      int row[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) row[i] = row_of(id[s][i]);
+      const int mine = (row[0] >= 0) + (row[1] >= 0) + (row[2] >= 0) + (row[3] >= 0);
+      if (__any_sync(0xffffffffu, mine)) {
+        int at = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, at, o); if (lane >= o) at += y; }
+        const int total = __shfl_sync(0xffffffffu, at, 31);
+        at += n - mine;
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+          if (row[i] >= 0) {
+            s_list[warp][at++] = ((unsigned)row[i] << 16) | (unsigned)(warp * PER_WARP + s * 128 + lane * 4 + i);
+            atomicAdd(&s_off[row[i] * SCATTER_WARPS + warp], 1);
+          }
+        n += total;
+      }
+    }
+    __syncthreads();
+    /* counts -> positions, by row and, within a row, by warp (which is by token); a lane per row */
+    if (warp == 0) {
+      int base = 0, found = 0;
+#pragma unroll 1
+      for (int rb = 0; rb < SCATTER_ROWS && rb < rows; rb += 32) {
+        int4 *cp = reinterpret_cast<int4 *>(s_off + (rb + lane) * SCATTER_WARPS);
+        const int4 c = cp[0], d = cp[1];
+        const int sum = c.x + c.y + c.z + c.w + d.x + d.y + d.z + d.w;
+        int at = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, at, o); if (lane >= o) at += y; }
+        const int total = __shfl_sync(0xffffffffu, at, 31);
+        at += base - sum;
+        s_begin[rb + lane] = at;
+        const unsigned some = __ballot_sync(0xffffffffu, sum > 0);
+        if (sum > 0) { s_rows[found + __popc(some & ((1u << lane) - 1u))] = (unsigned char)(rb + lane); s_some[rb + lane] = 1; }
+        int4 p, q;
+        p.x = at; p.y = p.x + c.x; p.z = p.y + c.y; p.w = p.z + c.z; q.x = p.w + c.w; q.y = q.x + d.x; q.z = q.y + d.y; q.w = q.z + d.z;
+        cp[0] = p; cp[1] = q;
+        base += total; found += __popc(some);
+      }
+      if (lane == 0) { s_begin[min(SCATTER_ROWS, (rows + 31) / 32 * 32)] = base; s_matched = found; }
+    }
+    __syncthreads();
+    /* every warp places its list; s_off[row, warp] moves on with it */
+    for (int i0 = 0; i0 < n; i0 += 32) {
+      const bool have = i0 + lane < n;
+      const unsigned e = have ? s_list[warp][i0 + lane] : 0xffffffffu;
+      const unsigned peers = __match_any_sync(0xffffffffu, e >> 16);
+      const int before = __popc(peers & ((1u << lane) - 1u));
+      int *slot = &s_off[(e >> 16) * SCATTER_WARPS + warp];
+      int at = 0;
+      if (have) { at = *slot; s_tok[at + before] = (unsigned short)(e & 0xffffu); }
+      __syncwarp();
+      if (have && before == 0) *slot = at + __popc(peers);
+      __syncwarp();
+    }
+    __syncthreads();
+    auto token_row = [&](int m) {
+      long long rem = c0 + s_tok[m];
+      if (MODE) return src + rem * a.tok_src[0];
+      const float *p = src;
+      for (int d = 0; d < a.ntok; d++) { const long long x = rem % a.tok_ext[d]; rem /= a.tok_ext[d]; p += x * a.tok_src[d]; }
+      return p;
+    };
+    const int matched = s_matched;
+    /* the source rows of the commonest words are requested from memory beforehand: their sum is one serial chain */
+    if (MODE) {
+      const unsigned lines = ((unsigned)nf + 31) / 32;
+      for (int k = 0; k < matched; k++) {
+        const int m0 = s_begin[s_rows[k]], m1 = s_begin[s_rows[k] + 1];
+        if (m1 - m0 <= SCATTER_DEEP) continue;
+        for (unsigned i = threadIdx.x; i < (unsigned)(m1 - m0) * lines; i += SCATTER_THREADS) {
+          const unsigned m = i / lines;
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(token_row(m0 + (int)m) + f_begin + (i - m * lines) * 32));
+        }
+      }
+    }
+    for (unsigned item = warp; item < (unsigned)(matched * segs); item += SCATTER_WARPS) {
+      const unsigned k = item / (unsigned)segs;
+      const int r = s_rows[k], f = (int)(item - k * segs) * 128 + (MODE == 2 ? lane * 4 : lane);
+      const int m0 = s_begin[r], m1 = s_begin[r + 1];
+      float *orow = out + r * a.out_vstride;
+      if (MODE == 2) {
+        if (f >= nf) continue;
+        float4 *op = reinterpret_cast<float4 *>(orow + f_begin + f);
+        float4 acc = c0 == 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : *op;
+        for (int m = m0; m < m1; m += SCATTER_DEEP) {
+          float4 x[SCATTER_DEEP];
+#pragma unroll
+          for (int i = 0; i < SCATTER_DEEP; i++) if (m + i < m1) x[i] = __ldg(reinterpret_cast<const float4 *>(token_row(m + i) + f_begin + f));
+#pragma unroll
+          for (int i = 0; i < SCATTER_DEEP; i++) if (m + i < m1) { acc.x += x[i].x; acc.y += x[i].y; acc.z += x[i].z; acc.w += x[i].w; }
+        }
+        *op = acc;
+      } else {
+        /* four features 32 apart per lane */
+        long long oo[4], so[4];
+        float acc[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          feature(f + j * 32, &oo[j], &so[j]);
+          acc[j] = (c0 == 0 || f + j * 32 >= nf) ? 0.0f : orow[oo[j]];
+        }
+        constexpr int DEEP = MODE ? 4 : 1;
+        for (int m = m0; m < m1; m += DEEP) {
+          float x[DEEP][4];
+#pragma unroll
+          for (int i = 0; i < DEEP; i++)
+            if (m + i < m1) {
+              const float *p = token_row(m + i);
+#pragma unroll
+              for (int j = 0; j < 4; j++) if (f + j * 32 < nf) x[i][j] = __ldg(p + so[j]);
+            }
+#pragma unroll
+          for (int i = 0; i < DEEP; i++)
+            if (m + i < m1) {
+#pragma unroll
+              for (int j = 0; j < 4; j++) if (f + j * 32 < nf) acc[j] += x[i][j];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) if (f + j * 32 < nf) orow[oo[j]] = acc[j];
+      }
+    }
+    __syncthreads();
+  }
+  if (s_distinct) return;
+  for (int r = warp; r < rows; r += SCATTER_WARPS) {
+    int last = r;
+    for (int r2 = r + 1; r2 < rows; r2++) if (s_ar[r2] == s_ar[r]) last = r2;
+    if (last == r || !s_some[last]) continue;
+    float *to = out + r * a.out_vstride;
+    const float *from = out + last * a.out_vstride;
+    if (MODE == 2) {
+#pragma unroll 4
+      for (int f = lane * 4; f < nf; f += 128) *reinterpret_cast<float4 *>(to + f_begin + f) = *reinterpret_cast<const float4 *>(from + f_begin + f);
+    } else for (int f = lane; f < nf; f += 32) { long long oo, so; feature(f, &oo, &so); to[oo] = from[oo]; }
   }
 }
 

@@ -17,6 +17,8 @@ def numbering(kind, vocab, rng):
         return a * 3 - 20
     if kind == 'permuted':
         return rng.permutation(vocab).astype(np.float32)
+    if kind == 'runs':
+        return a // 3
     if kind == 'repeated':
         a[vocab // 2:] = a[:vocab - vocab // 2]
         if vocab > 4:
@@ -25,10 +27,10 @@ def numbering(kind, vocab, rng):
 
 
 SIZES = [(1, 4, 1, 1), (5, 7, 1, 3), (64, 64, 2, 33), (65, 96, 1, 4097), (130, 768, 3, 50), (1000, 1604, 1, 17), (257, 1028, 2, 100),
-         (40, 128, 1, 9000), (33, 20, 1, 700), (70, 36, 1, 1500)]
+         (40, 128, 1, 9000), (33, 20, 1, 700), (70, 36, 1, 1500), (20000, 12, 1, 300)]
 
 
-@pytest.mark.parametrize('kind', ['plain', 'shifted', 'permuted', 'repeated'])
+@pytest.mark.parametrize('kind', ['plain', 'shifted', 'permuted', 'repeated', 'runs'])
 @pytest.mark.parametrize('vocab,dim,batch,tokens', SIZES, ids=str)
 def test_lookup_and_gradient(kernels, vocab, dim, batch, tokens, kind):  # noqa: F811
     rng = np.random.default_rng([vocab, dim, tokens])
