@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(SCATTER_THREADS, 4) pb200_scatter_rows(const S
   __shared__ __align__(16) int s_off[SCATTER_ROWS * SCATTER_WARPS];   /* matches of (row, warp): their number, then where they go in s_tok */
   __shared__ int s_begin[SCATTER_ROWS + 1];                       /* where those of the row begin */
   __shared__ unsigned char s_rows[SCATTER_ROWS];                  /* rows with matches */
-  __shared__ int s_matched, s_distinct;
+  __shared__ int s_matched;
   __shared__ unsigned char s_some[SCATTER_ROWS];                  /* rows that had matches in any chunk */
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long v0 = (long long)blockIdx.x * a.rows_per_block;
@@ -387,14 +387,11 @@ __global__ void __launch_bounds__(SCATTER_THREADS, 4) pb200_scatter_rows(const S
     s_ar[threadIdx.x] = (int)threadIdx.x < rows ? a.arange[v0 + threadIdx.x] : __int_as_float(0x7fc00000);
     s_some[threadIdx.x] = 0;
   }
-  if (threadIdx.x == 0) s_distinct = 1;
   __syncthreads();
   const float ar0 = s_ar[0];
   bool consecutive = truncf(ar0) == ar0 && fabsf(ar0) < 8388608.0f;        /* differences of such values are exact */
   if ((int)threadIdx.x < rows) consecutive &= s_ar[threadIdx.x] == ar0 + (float)threadIdx.x;
   consecutive = __syncthreads_and(consecutive ? 1 : 0) != 0;
-  if (!consecutive && (int)threadIdx.x < rows)
-    for (int r = 0; r < (int)threadIdx.x; r++) if (s_ar[r] == s_ar[threadIdx.x]) s_distinct = 0;
   /* the last row of the token's value */
   auto row_of = [&](float x) {
     if (consecutive) { const float dlt = x - ar0; return dlt >= 0.0f && dlt < (float)rows && ar0 + dlt == x && truncf(dlt) == dlt ? (int)dlt : -1; }
@@ -558,7 +555,10 @@ __global__ void __launch_bounds__(SCATTER_THREADS, 4) pb200_scatter_rows(const S
     }
     __syncthreads();
   }
-  if (s_distinct) return;
+  if (consecutive) return;
+  bool repeats = false;
+  if ((int)threadIdx.x < rows) for (int r = 0; r < (int)threadIdx.x; r++) repeats |= s_ar[r] == s_ar[threadIdx.x];
+  if (!__syncthreads_or(repeats ? 1 : 0)) return;
   for (int r = warp; r < rows; r += SCATTER_WARPS) {
     int last = r;
     for (int r2 = r + 1; r2 < rows; r2++) if (s_ar[r2] == s_ar[r]) last = r2;
