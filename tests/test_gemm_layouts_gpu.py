@@ -42,8 +42,9 @@ def test_bf16_operands(kernels, m, n, k, a_kfast, b_kfast, pad):  # noqa: F811
 
 
 @pytest.mark.parametrize('a_kfast,b_kfast', [(True, False), (False, False), (False, True)])
-def test_bf16_operands_of_cta_pairs(kernels, a_kfast, b_kfast):  # noqa: F811
-    """Enough 256 x 256 tiles and k for CTA pairs, with a remainder on every axis."""
+def test_bf16_operands_of_cta_pairs(kernels, monkeypatch, a_kfast, b_kfast):  # noqa: F811
+    """CTA pairs, forced: by estimated time sizes this small take single CTAs.  A remainder on every axis."""
+    monkeypatch.setenv('POLY_B200_TC_CTAS', '2')
     run_bf16(kernels, 2312, 2184, 1048, a_kfast, b_kfast, 0)
 
 
@@ -144,17 +145,23 @@ def test_f32_operands_rounded_to_bf16(kernels, m, n, k, a_kfast, b_kfast, pad): 
 
 
 @pytest.mark.parametrize('relu', [0, 1])
-@pytest.mark.parametrize('m,n,k,pitch,offset', [(2312, 2185, 72, 2185, 0), (129, 18945, 64, 18950, 4), (2561, 1799, 1048, 1803, 12)], ids=str)
-def test_rows_written_line_by_line(kernels, m, n, k, pitch, offset, relu):  # noqa: F811
-    """CTA pairs whose result rows start anywhere: every offset of a row in its 128-byte line, parts of a tile with
-    one column and none, ragged rows; what lies between the rows stays as it was."""
+@pytest.mark.parametrize('m,n,k,pitch,offset,b_kfast', [(2312, 2185, 72, 2185, 0, True), (129, 18945, 64, 18950, 4, True), (2561, 1799, 1048, 1803, 12, True),
+                                                        (2312, 2185, 72, 2185, 0, False), (2620, 51237, 16, 51237, 8, True)], ids=str)
+def test_rows_written_line_by_line(kernels, monkeypatch, m, n, k, pitch, offset, b_kfast, relu):  # noqa: F811
+    """CTA pairs (forced, with the 74 tiles that this way of writing asks for) whose result rows start anywhere: every offset of
+    a row in its 128-byte line, parts of a tile with one column and none, ragged rows; what lies between the rows stays as
+    it was.  The largest result (537 MB) is written with streaming stores."""
+    monkeypatch.setenv('POLY_B200_TC_CTAS', '2')
     rng = np.random.default_rng([m, n, k])
     a, b = bf16(rng.standard_normal((m, k))), bf16(rng.standard_normal((n, k)))
+    mb, (b_sn, b_sk) = stored(b, b_kfast, 0, rng, bits)
     c = kernels.put(np.full((m, pitch), 7, np.float32), offset)
-    assert kernels.c.poly_b200_gemm(m, n, k, kernels.put(bits(a)), k, 1, kernels.put(bits(b)), 1, k, c, pitch, None, relu, 1) == 0, kernels.error()
-    got, want = kernels.get(c, (m, pitch)), a.astype(np.float64) @ b.T.astype(np.float64)
+    assert kernels.c.poly_b200_gemm(m, n, k, kernels.put(bits(a)), k, 1, kernels.put(mb), b_sk, b_sn, c, pitch, None, relu, 1) == 0, kernels.error()
+    got = kernels.get(c, (m, pitch))
     assert np.all(got[:, n:] == 7)
-    assert_close(got[:, :n], np.maximum(want, 0) if relu else want, 1e-4, f'{m} {n} {k}')
+    for r in range(0, m, 500):
+        want = a[r:r + 500].astype(np.float64) @ b.T.astype(np.float64)
+        assert_close(got[r:r + 500, :n], np.maximum(want, 0) if relu else want, 1e-4, f'{m} {n} {k} from row {r}')
 
 
 @pytest.mark.parametrize('a_kfast,b_kfast', [(True, False), (False, True)])
@@ -227,3 +234,29 @@ def test_f32_nan_of_any_payload(kernels):  # noqa: F811
     want = np.zeros((m, n), bool)
     want[[3, 700], :] = want[:, 77] = True
     assert np.array_equal(np.isnan(kernels.get(c, (m, n))), want)
+
+
+@pytest.mark.parametrize('arith', ['f32', 'policy', 'bf16'])
+@pytest.mark.parametrize('shared_b', [False, True])
+@pytest.mark.parametrize('a_kfast,b_kfast', [(True, False), (True, True), (False, False), (False, True)])
+def test_batches(kernels, monkeypatch, a_kfast, b_kfast, shared_b, arith):  # noqa: F811
+    """Two batch axes, the second operand the same for one of them or not: the parts, copies and views of every batch entry."""
+    if arith == 'f32':
+        monkeypatch.setenv('POLY_B200_FP32', 'tcp')
+    kernels.c.poly_b200_set_gemm_policy(int(arith == 'policy'))
+    rng = np.random.default_rng([a_kfast, b_kfast, shared_b])
+    h, t, m, n, k = 2, 3, 136, 72, 40
+    a, b = rng.standard_normal((t, h, m, k)).astype(np.float32), rng.standard_normal((t, 1 if shared_b else h, n, k)).astype(np.float32)
+    if arith != 'f32':
+        a, b = bf16(a), bf16(b)
+    want = a.astype(np.float64) @ b.astype(np.float64).transpose(0, 1, 3, 2)
+    conv = bits if arith == 'bf16' else (lambda x: x)
+    ma, mb = (conv(x if kfast else x.transpose(0, 1, 3, 2)) for x, kfast in ((a, a_kfast), (b, b_kfast)))
+    a_sm, a_sk = (k, 1) if a_kfast else (1, m)
+    b_sn, b_sk = (k, 1) if b_kfast else (1, n)
+    b_h, b_t = (0, n * k) if shared_b else (n * k, h * n * k)
+    c = kernels.put(np.zeros((t, h, m, n), np.float32))
+    kernels.launch(f'//PB200 1\n//kind gemm\n//nparams 3\n//params 0 1 2 -1\n//offsets 0 0 0 0\n//relu 0\n//dtype {"bf16" if arith == "bf16" else "f32"}\n'
+                   f'//naxes 5\n//axis0 b {h} {m * n} {m * k} {b_h} 0\n//axis1 b {t} {h * m * n} {h * m * k} {b_t} 0\n//axis2 m {m} {n} {a_sm} 0 0\n'
+                   f'//axis3 n {n} 1 0 {b_sn} 0\n//axis4 k {k} 0 {a_sk} {b_sk} 0\n//numel {h * t * m * n}\n', 'batches', [c, kernels.put(ma), kernels.put(mb)])
+    assert_close(kernels.get(c, (t, h, m, n)), want, 1e-5 if arith == 'f32' else 1e-4, arith)
