@@ -339,7 +339,88 @@ static SgemmFn pick_vec(bool va, bool vb) {
   return pb200_sgemm<AK, BKm, false, false>;
 }
 
-/* Small problems: 128 x 128 tiles would leave most SMs idle (the 256 x 784 x 512 and 256 x 512 x 10 layers of an
+/* Small problems with a short k axis: 32 x 32 tiles, 256 threads, 2 x 2 results per thread, any strides; every fourth k has
+ * a sum of its own (as in the kernel below: half the rounding error of one sum in k order).  Bound by shared memory, two reads per two
+ * multiply-adds, but it starts and ends quickly and its blocks share SMs.  Launched plainly: with programmatic dependence its blocks
+ * start where slots come free, several on one SM beside idle ones (1297 x 67 x 761 27 -> 50 us). */
+#define TB 32
+__global__ void __launch_bounds__(256, 3) pb200_sgemm_tile32(const SgemmArgs g) {
+  __shared__ float As[2][TB][TB + 1];      /* [k][m] */
+  __shared__ float Bs[2][TB][TB + 1];      /* [k][n] */
+  long long oa = 0, ob = 0, oc = 0, ox = 0;
+  {
+    int rem = blockIdx.z;
+    for (int i = 0; i < g.nb; i++) {
+      const int x = rem % g.bext[i]; rem /= g.bext[i];
+      oa += x * g.a_sb[i]; ob += x * g.b_sb[i]; oc += x * g.c_sb[i]; ox += x * g.x_sb[i];
+    }
+  }
+  const float *__restrict__ A = g.A + oa;
+  const float *__restrict__ B = g.B + ob;
+  const int m0 = blockIdx.y * TB, n0 = blockIdx.x * TB;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  /* element e of a 32 x 32 tile: consecutive threads along the operand's contiguous axis */
+  const bool a_kfast = g.a_sk == 1, b_kfast = g.b_sk == 1 && g.b_sn != 1;
+  float ra[4], rb[4];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int e = tid + i * 256;
+      const int ka = a_kfast ? (e & 31) : (e >> 5), ma = a_kfast ? (e >> 5) : (e & 31);
+      const int kb = b_kfast ? (e & 31) : (e >> 5), nb = b_kfast ? (e >> 5) : (e & 31);
+      ra[i] = (m0 + ma < g.M && k0 + ka < g.K) ? A[(long long)(m0 + ma) * g.a_sm + (long long)(k0 + ka) * g.a_sk] : 0.0f;
+      rb[i] = (n0 + nb < g.N && k0 + kb < g.K) ? B[(long long)(k0 + kb) * g.b_sk + (long long)(n0 + nb) * g.b_sn] : 0.0f;
+    }
+  };
+  auto stash = [&](int buf) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int e = tid + i * 256;
+      const int ka = a_kfast ? (e & 31) : (e >> 5), ma = a_kfast ? (e >> 5) : (e & 31);
+      const int kb = b_kfast ? (e & 31) : (e >> 5), nb = b_kfast ? (e >> 5) : (e & 31);
+      As[buf][ka][ma] = ra[i];
+      Bs[buf][kb][nb] = rb[i];
+    }
+  };
+  float acc[4][2][2] = {};                 /* sums of every fourth k */
+  fetch(0);
+  stash(0);
+  __syncthreads();
+  const int nk = (g.K + TB - 1) / TB;
+  for (int kt = 0; kt < nk; kt++) {
+    const int cur = kt & 1;
+    if (kt + 1 < nk) fetch((kt + 1) * TB);
+#pragma unroll
+    for (int k = 0; k < TB; k++) {
+      const float a0 = As[cur][k][ty * 2], a1 = As[cur][k][ty * 2 + 1];
+      const float b0 = Bs[cur][k][tx * 2], b1 = Bs[cur][k][tx * 2 + 1];
+      float (&p)[2][2] = acc[k & 3];
+      p[0][0] = fmaf(a0, b0, p[0][0]); p[0][1] = fmaf(a0, b1, p[0][1]);
+      p[1][0] = fmaf(a1, b0, p[1][0]); p[1][1] = fmaf(a1, b1, p[1][1]);
+    }
+    if (kt + 1 < nk) stash(cur ^ 1);
+    __syncthreads();
+  }
+  float *__restrict__ C = g.C + oc;
+  const float *__restrict__ X = g.has_x ? g.X + ox : nullptr;
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const int m = m0 + ty * 2 + i;
+    if (m >= g.M) continue;
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+      const int n = n0 + tx * 2 + j;
+      if (n >= g.N) continue;
+      float t = __fmul_rn((acc[0][i][j] + acc[1][i][j]) + (acc[2][i][j] + acc[3][i][j]), g.alpha);
+      if (X) t = t + X[(long long)m * g.x_sm + (long long)n * g.x_sn];
+      if (g.relu) t = (0.0f < t) ? t : 0.0f;
+      C[(long long)m * g.c_sm + (long long)n * g.c_sn] = t;
+    }
+  }
+}
+
+
+/* Small problems with a longer k axis: 128 x 128 tiles would leave most SMs idle (the 256 x 784 x 512 and 256 x 512 x 10 layers of an
  * MLP are 8 and 2 of them), so 64 x 64 tiles, and the k axis of a tile split twice: between the 2, 4 or 8 CTAs of a
  * cluster, and between the four 64-thread groups of a CTA, which take every fourth quad of k.  A thread then still
  * has 8 x 8 results (16 128-bit shared-memory loads per 256 multiply-adds; with 2 x 2 results shared memory was the
@@ -507,22 +588,38 @@ static int sgemm_launch(const SgemmArgs &g, long long nbatch, cudaStream_t strea
     for (int i = 0; i < nb; i++) if (sb[i] & 3) return false;
     return true;
   };
-  /* fewer large tiles than half the SMs: small tiles, their k axis split between as many CTAs as keep the SMs busy.
-   * Estimated in clocks: a slab of a tile, the start and the two reductions of a CTA. */
+  /* Fewer large tiles than half the SMs: the 32 x 32 kernel, or 64 x 64 tiles with their k axis split over 1 to 8 CTAs,
+   * whichever is estimated to take less time.  The estimates, in microseconds per call among other calls, were fitted to 260 shapes
+   * (M, N to 16384, K 32 to 1500, three operand orders): 5 % off (rms) for the first, 3 % for the second.
+   * 32 x 32: a slab of 32 k, more where an SM has several blocks.  64 x 64: rounds of as many clusters as fit the GPU at
+   * once (33 of four CTAs, 15 of eight: a cluster stays within a part of the chip), each a start with its reductions and a slab per 32 k,
+   * dearer with k-contiguous B and with operands copied 4 bytes at a time.  300 other shapes take 0.77 of
+   * the time of the first kernel alone; the second alone took 0.83, and up to twice the first's on a third of them (219 x 547 x 156 17.6 us as
+   * 36 clusters of four, 8.5 in 32 x 32 tiles; 256 x 512 x 784 14.8 as 32 clusters of four, 28.7). */
   {
     const long long big = (long long)((g.M + BM - 1) / BM) * ((g.N + BN - 1) / BN) * nbatch;
     const long long tn = (g.N + SB - 1) / SB, tm = (g.M + SB - 1) / SB, tiles = tm * tn * nbatch;
     if (big < 74 && tm <= 65535 && nbatch <= 65535) {
-      const long long slabs = ((long long)g.K + SK - 1) / SK;
-      int n_split = 1;
-      long long best = -1;
-      for (int s = 1; s <= 8; s *= 2) {
-        const long long cost = ((tiles * s + 147) / 148) * ((slabs + s - 1) / s * 1200 + (s > 1 ? 4500 : 3500));
-        if (best < 0 || cost < best) { best = cost; n_split = s; }
-      }
       const bool ak = g.a_sk == 1, bk = g.b_sk == 1 && g.b_sn != 1;
       const bool wa = (ak || g.a_sm == 1) && aligned(g.A, ak ? g.a_sm : g.a_sk, g.a_sb, g.nb);
       const bool wb = (bk || g.b_sn == 1) && aligned(g.B, bk ? g.b_sn : g.b_sk, g.b_sb, g.nb);
+      const long long slabs = ((long long)g.K + SK - 1) / SK;
+      const dim3 small_grid((unsigned)((g.N + TB - 1) / TB), (unsigned)((g.M + TB - 1) / TB), (unsigned)nbatch);
+      const double per_sm = (double)(((long long)small_grid.x * small_grid.y * nbatch + 147) / 148);
+      double best = 3.8 + (double)slabs * (1.0 + (per_sm > 1 ? 0.5 * (per_sm - 1) : 0) + (per_sm > 3 ? 0.24 * (per_sm - 3) : 0));
+      int n_split = 0;
+      const double slab = 1.31 + (bk ? 0.52 : 0) + (wa ? 0 : 0.34) + (wb ? 0 : 0.43);
+      static const struct { int s, fit; double start; } forms[4] = {{1, 148, 2.3}, {2, 74, 5.0}, {4, 33, 4.3}, {8, 15, 3.8}};
+      for (auto &f : forms) {
+        const double t = 1.0 + (double)((tiles + f.fit - 1) / f.fit) * (f.start + (double)((slabs + f.s - 1) / f.s) * slab);
+        if (t < best) { best = t; n_split = f.s; }
+      }
+      if (n_split == 0) {
+        pb200_sgemm_tile32<<<small_grid, 256, 0, stream>>>(g);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) { pb_set_error("sgemm launch: %s", cudaGetErrorString(e)); return -1; }
+        return 0;
+      }
       const dim3 grid((unsigned)tn, (unsigned)tm, (unsigned)nbatch);
       if (ak) return bk ? small_launch<true, true>(g, grid, n_split, wa, wb, stream) : small_launch<true, false>(g, grid, n_split, wa, wb, stream);
       return bk ? small_launch<false, true>(g, grid, n_split, wa, wb, stream) : small_launch<false, false>(g, grid, n_split, wa, wb, stream);

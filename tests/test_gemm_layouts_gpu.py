@@ -109,14 +109,14 @@ def test_rows_of_float32_off_the_16_byte_grid(kernels, m, n, k, relu):  # noqa: 
         assert_close(got[r:r + 500], np.maximum(want[r:r + 500], 0) if relu else want[r:r + 500], 1e-4, f'{m} {n} {k} from row {r}')
 
 
-SMALL = [(1, 1, 1), (256, 10, 512), (64, 64, 32), (65, 63, 33), (3, 200, 5000), (100, 1, 77), (1, 100, 64), (256, 512, 784), (500, 900, 100)]
+SMALL = [(1, 1, 1), (256, 10, 512), (64, 64, 32), (65, 63, 33), (3, 200, 5000), (100, 1, 77), (1, 100, 64), (256, 512, 784), (500, 900, 100), (640, 420, 288)]
 
 
 @pytest.mark.parametrize('pad', [0, 4, 3])
 @pytest.mark.parametrize('a_kfast,b_kfast', [(True, False), (True, True), (False, False), (False, True)])
 @pytest.mark.parametrize('m,n,k', SMALL, ids=str)
 def test_small_f32(kernels, m, n, k, a_kfast, b_kfast, pad):  # noqa: F811
-    """One to eight CTAs per tile, slabs of k that are missing, partial or past the end, every operand order and
+    """Tiles of 32 and of 64, one to eight CTAs per tile, slabs of k that are missing, partial or past the end, every operand order and
     alignment; the sums are float32 ones in another order than float64's, far inside 1e-5 at these K."""
     rng = np.random.default_rng([m, n, k, pad])
     a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
