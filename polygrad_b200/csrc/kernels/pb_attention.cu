@@ -575,7 +575,7 @@ pb200_flash_attn2(const __grid_constant__ CUtensorMap map_q, const __grid_consta
          * them through its 4 KB of the P tile (idle between the previous block's product and this block's
          * probabilities): the first 32 keys copied there asynchronously, the others held in registers meanwhile.
          * Read by each thread along its own row, 32 rows per instruction, 1 x 25 x 2048 x 64 with a position bias
-         * took 249 us, most of it in the L1's line lookups; 188 like this (pb200_attn_prepare included). */
+         * took 249 us, most of it in the L1's line lookups; 185 like this (pb200_attn_prepare included). */
         if (it > 0 && !__all_sync(0xffffffffu, mbar_wait(bar_o, (it - 1) & 1u, &abort_flag, 18))) { ok = false; break; }
         const uint32_t stg = s_p + half * 16384 + quarter * 4096;
         const int sub = lane & 7, rr = lane >> 3;
@@ -873,7 +873,7 @@ __global__ void __launch_bounds__(256) pb200_mask_tiles(const float *mask, long 
  * mask's tiles; each of the others rounds 128 rows of one head of q, k and v to bfloat16 (same [B][T][H][64] layout)
  * and bounds the norms of the rounded q and k rows while they are in registers.  Bound by memory (4 bytes read, 2
  * written per element).  (Three conversions, the bounds and the classification were five
- * launches: 8 x 12 x 1024 x 64 with a causal mask took 115.5 us in all, 89 like this.) */
+ * launches: 8 x 12 x 1024 x 64 with a causal mask took 115 us in all, 85 like this.) */
 struct PrepareArgs {
   const float *src[3]; __nv_bfloat16 *dst[3];
   int H, T, nblk; long long D;
@@ -1042,11 +1042,11 @@ int pb_attention_error(void) {
 /* at most 64 key blocks: the set of processed blocks is a 64-bit mask */
 bool pb_attention_supported(long long T, long long hd) { return hd == AT_HD && T >= AT_BK && T % AT_BK == 0 && T / AT_BK <= 64; }
 
-/* q, k, v: bf16 through strides; mask fp32 [T x T] through strides; out fp32 or bf16 (out_bf16)
- * at element offsets Σ batch_i*o_sb[i] + row*o_sm + d. */
 /* POLY_B200_ATTN_SKIP=0: no key block is left out */
 static bool attn_skips() { const char *e = getenv("POLY_B200_ATTN_SKIP"); return !(e && e[0] == '0'); }
 
+/* q, k, v: bf16 through strides; mask fp32 [T x T] through strides; out fp32 or bf16 (out_bf16)
+ * at element offsets Σ batch_i*o_sb[i] + row*o_sm + d. */
 int pb_attention_launch(const PbAttnOperand &q, const PbAttnOperand &k, const PbAttnOperand &v,
                         const float *mask, long long mask_sq, long long mask_sk,
                         float scale, void *out, bool out_bf16, int nb, const int *bext, const long long *o_sb, long long o_sm,

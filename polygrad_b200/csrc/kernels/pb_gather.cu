@@ -19,7 +19,7 @@
  * Either way the result is the reference's.  (Checking first and copying after
  * cost two dependent kernels with a single block in the first: 8192 tokens of a
  * 50257 x 768 table took 61 us, of which the copy, a block per token and an element
- * per thread, was 51; 13-14 us like this.)
+ * per thread, was 51; 14 us like this.)
  *
  * HBM traffic is the table rows read plus the output rows written.
  */
@@ -330,7 +330,7 @@ PbAotProgram *pb_make_gather(const PbHeader &h, std::string &err) {
  *
  * HBM traffic: the output written once, the ids read once per block (from L2), the matching source rows.  8192
  * tokens (ids distributed as words in text) into a 50257 x 768 table: 1000 us with blocks of 16 rows that compared
- * one id at a time with all of them, sorted the matches by insertion on one thread and added one load at a time; 67 us like this, of which the zeros
+ * one id at a time with all of them, sorted the matches by insertion on one thread and added one load at a time; 65 us like this, of which the zeros
  * are 33 (4.7 TB/s) and the longest chains (a word 272 times) most of the rest. */
 struct ScatterArgs {
   float *out; const float *ids; const float *arange; const float *src;

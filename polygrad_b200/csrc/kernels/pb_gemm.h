@@ -19,8 +19,8 @@ enum { PB_F32 = 0, PB_BF16 = 1, PB_F16 = 2 };      /* storage type of a contract
  * touch global memory.  pb_grid_release() lets the next such launch do the same; called at the start, since a
  * kernel's blocks must all have started before the next one's do.  A kernel launched like this calls
  * pb_grid_wait() on every path.  197 x 2304 x 768 under the bfloat16 policy, a copy
- * and a contraction: 14.3 us one after the other, 11.1 like this.  (Not released early in front of the attention kernel: its
- * blocks would be dealt out as slots come free, unevenly: 8 x 12 x 1024 x 64 89 -> 92 us.) */
+ * and a contraction: 14.3 us one after the other, 11.2 like this.  (Not for kernels of which an SM holds several blocks, unless they are many:
+ * blocks are dealt out as slots come free, unevenly.  8 x 12 x 1024 x 64 attention released early 89 -> 92 us, a small contraction 27 -> 50.) */
 template <class F, class... Args>
 static inline cudaError_t pb_launch_chained(F *kernel, dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, unsigned cluster, Args... args) {
   cudaLaunchConfig_t cfg = {};

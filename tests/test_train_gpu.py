@@ -149,7 +149,7 @@ def test_gpt2_train_steps_with_backward_kernels_cut(ref_lib, gpu, monkeypatch, o
     gradient's contraction.  Same tolerances as the uncut run.  `sgd_tensor_cores` also sends every
     float32 contraction the tensor-core kernel accepts through it (three tf32 products, operands split --
     and, where their rows are the contiguous axis, transposed -- on the way; scaled sums included), as
-    happens by default from 2^30 multiply-adds."""
+    happens by default to large ones."""
     monkeypatch.setenv('POLY_B200_OUTLINE_MIN_WORK', '0')
     if route:
         monkeypatch.setenv('POLY_B200_FP32', route)
